@@ -58,8 +58,10 @@ def listed():
         dict(name="prefill-7b-fp16-8192", kind="prefill", H=4096, I=11008, r=128, B=8192, L=1, dtype="fp16", density=0.10, act="relu", gate=True, rule="naive"),
         # norms, attention and output projection of four decoder layers, 4000 tokens of context
         dict(name="glue-3b-fp16-ctx4000", kind="glue", heads=24, kv=8, hd=128, H=3072, ctx=4000, max_len=4096, L=4, dtype="fp16"),
-        # a whole decoder: eight layers of the 3B shape, logits of four tokens behind a 200-token prompt
-        dict(name="model-3b-fp16-8l", kind="model", H=3072, I=8192, r=64, heads=24, kv=8, hd=128, vocab=128256, L=8, prompt=200, max_len=1024, dtype="fp16", density=0.20, act="silu"),
+        # a whole decode call, embedding to logits, of four tokens behind a 200-token prompt.  One decoder layer of the 3B shape:
+        # with random weights an inactive neuron is not a small one, so a single rounding that moves a neuron across the
+        # threshold of a later layer moves the logits by several per cent, and the call could be compared with nothing
+        dict(name="model-3b-fp16-1l", kind="model", H=3072, I=8192, r=64, heads=24, kv=8, hd=128, vocab=128256, L=1, prompt=200, max_len=1024, dtype="fp16", density=0.20, act="silu"),
     ]
 
 
@@ -347,9 +349,10 @@ def work(case):
 
 def tolerance(case):
     """32-bit sums in another order; in 16 bits one rounding of the activations and of the result on either side.  Masks are
-    whole values and reproducible bit for bit; the model's logits carry the roundings of all its layers."""
+    whole values and reproducible bit for bit.  The model's logits differ by 8e-4 when its attention, norms and projections
+    round in another order."""
     if case["kind"] == "model":
-        return {"rel": 2e-2}
+        return {"rel": 3e-3}
     if case["dtype"] == "fp32":
         return {"rel": 1e-5}
     return {"rel": 1e-2 if case["dtype"] == "bf16" else 2e-3}
