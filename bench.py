@@ -860,7 +860,7 @@ def prefill_measure(args, dev):
         del cw, dp, comb, scratch
     top = sweep["1.00"]
     return {"workload": w.name, "tflops": top["tflops"], "ms_per_step": top["ms"], "rows": T, "steps": steps,
-            "roofline": {"kernel": "k_umma_gemm", "bound": "tensor", "achieved": top["tflops"], "peak": peak,
+            "roofline": {"kernel": "k_pair_gemm", "bound": "tensor", "achieved": top["tflops"], "peak": peak,
                          "unit": "TFLOP/s", "frac": top["tflops"] / peak, "peak_source": peak_src, "traffic": None,
                          "flops_per_step": 6.0 * T * H * I},
             "k_sweep": sweep, "gpu_launches": 3 * steps,

@@ -189,7 +189,7 @@ int stx_mlp_scratch_bytes(int64_t B, int64_t H, int64_t K, size_t* bytes_out);
  * depends on B and H: a buffer that is reused for a call with a different B or H must have
  * the new call's leading region zeroed again first (cudaMemsetAsync on the same stream).  Row blocks of 9 and more in
  * fp16/bf16 (prefill) run as two tcgen05 tensor-core GEMMs instead and keep their
- * activation matrix and a transposed copy of the down rows behind those regions.         */
+ * activation matrix and the partial sums of a split contraction behind those regions.    */
 int stx_sparse_mlp_forward(const void* x, int64_t B, int64_t H, const void* concat_w,
                            const void* down_packed, int64_t K, void* down_buf,
                            void* combined_buf, int act, int has_gate, int dtype,

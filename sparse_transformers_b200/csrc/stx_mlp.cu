@@ -367,7 +367,7 @@ extern "C" {
 int stx_mlp_scratch_bytes(int64_t B, int64_t H, int64_t K, size_t* bytes_out) {
   STX_CHECK_ARG(bytes_out && B > 0 && H > 0 && K >= 0, "stx_mlp_scratch_bytes: bad argument");
   // decode kernels' regions, then (row blocks of 9 and more) the tensor-core path's
-  // activation matrix and transposed down weight
+  // activation matrix and partial sums
   *bytes_out = decode_scratch_bytes(B, H, K) + (B >= STX_GEMM_MIN_ROWS ? prefill_scratch_bytes(B, H, K) : 0);
   return STX_OK;
 }

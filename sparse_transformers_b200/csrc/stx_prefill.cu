@@ -1,27 +1,35 @@
-// Sparse gated MLP over packed active rows for prefill-sized row blocks (hundreds of rows
-// and more): here the gathered weights really form a dense contraction, so it runs on the
-// 5th-generation tensor cores.
+// Sparse gated MLP over packed active rows for row blocks (9 rows and more) in fp16/bf16: here the
+// gathered weights form a dense contraction, so it runs on the 5th-generation tensor cores.
 //
-//   GEMM 1   [G | U] = X · [Wg ; Wu]^T      M = rows, N = K (twice), k = H
-//            epilogue: A = act(G) * U  -> fp16/bf16 scratch [rows, K8] (and combined_buf)
-//   GEMM 2   out = A · Wd                    M = rows, N = H, k = K
-//            (Wd: the packed down rows, transposed once per call to [H, K8] so that both
-//             operands of both GEMMs are K-major)
+//   GEMM 1   [G ; U] = [Wg ; Wu] · X^T      M = neurons (gate and up rows), N = tokens, k = H
+//            epilogue: A = act(G) * U -> fp16/bf16 scratch [tokens, K8] (and combined_buf)
+//   GEMM 2   out^T  = Wd^T · A^T            M = H, N = tokens, k = neurons
 //
-// One kernel, k_umma_gemm<T, MODE, MH>: per CTA MH (1 or 2) row halves of 128 and two 128-wide
-// B tiles (MODE 0: gate and up rows of the same 128 neurons; MODE 1: 256 output columns), so a
-// 64-wide k block of 64 KB feeds eight 128x128x16 MMAs; 64-wide k blocks.
-//   warp 0      producer: TMA tiled loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the A
-//               tile and one (MODE 1) or two (MODE 0: gate and up rows) B tiles into a ring of
-//               shared-memory stages, completion on mbarriers
-//   warp 1      allocates tensor memory and issues tcgen05.mma (cta_group::1, kind::f16,
-//               M=128, N=128, K=16) from one elected lane; accumulators live in TMEM (128 or
-//               256 columns); tcgen05.commit releases a stage / publishes the accumulator
-//   warps 2..5  epilogue: tcgen05.ld 32 lanes x 32 columns at a time, activation and product
-//               in registers, 16-byte stores
-// Edges are handled by TMA zero fill on loads and by masked stores.  Every CTA loads its own tiles.
-// Every mbarrier wait is bounded; on expiry the kernel records DEV_TIMEOUT and continues
-// with the same control flow (the result is then garbage) so that TMEM is always freed.
+// The weights are the M side and the tokens the N side: a few dozen tokens then cost an N of 32..128
+// and not a 128-row tile, an odd number of tokens is padded to the next 32 and not to 256, and the
+// packed down rows [K, H] are an M-major operand as they lie (the k-major form needs a transposed
+// copy of them on every call: 26 us of a 166 us layer at 64 tokens and K = 8700, 90 MB at K = 11008).
+//
+// One kernel, k_pair_gemm<T, MODE>: a cluster of two CTAs (one SM pair) works on tiles of 256 M rows
+// x N tokens with tcgen05.mma.cta_group::2 (M = 256): each CTA holds its 128 M rows of A and half of
+// the tokens, so the token operand crosses into shared memory once per pair.  The grid is one pair
+// per SM pair; a pair walks the tiles, two accumulators of 256 TMEM columns alternate, so that the
+// epilogue of a tile runs while the next one is multiplied.
+//   MODE 0: a CTA's 128 M rows are the gate rows (0..63) and the up rows (64..127) of the same 64
+//           neurons (fewer when the neurons are shared out evenly, see pf_plan())
+//   MODE 1: 128 columns of H, loaded as two [64 neurons][64 columns] boxes, M-major
+//   warps 0, 6, 7  producers: TMA tiled loads (128-byte swizzle) of a 64-wide k block per stage, one
+//               box of the stage each (gate / up rows or the two column boxes / tokens): a warp
+//               issues about one box per 85 ns, and three in a row made the issue the bottleneck
+//               (64 tokens, 8700 neurons of 4096: GEMM 1 57 -> 44 us).  Both CTAs' copies complete on the even CTA's barrier
+//   warp 1      even CTA: issues the MMAs from one lane; tcgen05.commit (multicast to both CTAs)
+//               releases a stage / publishes an accumulator.  Allocates and frees tensor memory.
+//   warps 2..5  epilogue: tcgen05.ld 32 lanes x 32 tokens; a warp's 32 lanes are neighbouring
+//               columns of the result, so every store is one contiguous 64- or 128-byte piece
+//               whatever the alignment of the row.
+// Edges are handled by TMA zero fill on loads and by masked stores; no load is multicast.
+// Every mbarrier wait is bounded; a role whose wait expired records DEV_TIMEOUT, stops, and the
+// others run out of their own waits in turn, so that TMEM is always freed.
 #include "stx_common.cuh"
 
 #include <cuda.h>
@@ -32,31 +40,37 @@
 
 namespace stx {
 
-constexpr int PF_BM = 128, PF_BN = 128, PF_BK = 64;
-constexpr int PF_THREADS = 192;
-constexpr uint32_t PF_TILE_BYTES = PF_BM * PF_BK * 2;  // 16 KB per operand tile
+constexpr int PF_BK = 64;
+constexpr int PF_THREADS = 256;
+constexpr int PF_TW = 128;                               // neurons of a MODE 0 tile (64 per CTA)
+constexpr int PF_HW = 256;                               // columns of H of a MODE 1 tile (128 per CTA)
+constexpr int PF_MAX_N = 256;                            // tokens of a tile
+constexpr int PF_MAX_STAGES = 12;
+constexpr uint32_t PF_A_BYTES = 128 * PF_BK * 2;         // a CTA's A tile of one stage
+constexpr uint32_t PF_XCH_BYTES = 2 * 2 * 2 * 16 * 32 * 4;  // [warp pair][buffer][g|u][16 tokens][32 lanes] fp32
+constexpr uint32_t PF_SMEM = 226 * 1024;
 constexpr uint32_t PF_WAIT_LIMIT = 1u << 22;
+constexpr int PF_GROUP = 8;                              // token tiles that walk the weights together
 
 struct PfArgs {
-  int M, N, Kd;        // output rows, output columns, contraction length
-  int up_off;          // MODE 0: row offset of the up block inside the concat weight (= K)
+  int M;               // tokens
+  int N;               // MODE 0: neurons K ; MODE 1: columns H
+  int Kd;              // contraction length: H ; K
+  int n_tok;           // tokens of a tile (multiple of 32)
+  int tok_tiles;
+  int pairs;           // SM pairs the tiles are shared out over
+  int even;            // MODE 0: share the neurons out evenly over whole waves (one token tile)
+  int splits;          // MODE 1: contraction splits
   int stages;
-  int stages_z;        // number of contraction splits (gridDim.z), 0/1 = none
-  void* a_out;         // MODE 0: activations [M, lda] ; MODE 1: output [M, ldo]
+  void* a_out;         // MODE 0: activations [M, ld_out] or null; MODE 1: output [M, ld_out]
   int ld_out;
   void* combined;      // MODE 0, optional: [M, 2K]
   int act;
   int* status;
   // Optional device-side count of valid rows of the packed weights (a weight cache's K): MODE 0
-  // writes zero activations for columns >= *k_dev and skips tiles wholly beyond it; MODE 1 stops
-  // its contraction at *k_dev (rounded up to a k-block, which MODE 0 filled with zeros).
+  // covers *k_dev neurons rounded up to a k-block, zeros beyond *k_dev; MODE 1 stops its contraction there.
   const int* k_dev;
-  // Optional split of the contraction over gridDim.z CTAs: CTA z takes an equal share of the k-blocks
-  // and writes its fp32 partial tile; the caller adds the partials.  MODE 1: part[z][M][ld_out].
-  // MODE 0: part[z][M][2*ld_part], gate sums in columns [0, N), up sums in [ld_part, ld_part + N)
-  // (the activation needs the complete sums, so it moves to the kernel that adds the partials).
-  float* part;
-  int ld_part;
+  float* part;         // MODE 1 with splits: part[split][M][ld_out], summed by the caller in split order
 };
 
 __device__ __forceinline__ uint32_t pf_smem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -66,11 +80,19 @@ __device__ __forceinline__ void pf_mbar_init(uint64_t* b, uint32_t n) {
 __device__ __forceinline__ void pf_expect_tx(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(pf_smem(b)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ uint32_t pf_mapa(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(pf_smem(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void pf_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ bool pf_try_wait(uint64_t* b, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(pf_smem(b)), "r"(parity)
@@ -84,34 +106,39 @@ __device__ __forceinline__ bool pf_wait(uint64_t* b, uint32_t parity) {
   }
   return false;
 }
-__device__ __forceinline__ void pf_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
+// bar: shared::cluster address of the even CTA's barrier
+__device__ __forceinline__ void pf_tma_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
           pf_smem(dst)),
-      "l"(map), "r"(pf_smem(bar)), "r"(c0), "r"(c1)
+      "l"(map), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-// K-major operand tile with 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t pf_smem_desc(const void* tile) {
+// Operand tile with 128-byte swizzle.  K-major: rows of 64 k elements, 8-row groups 1024 bytes apart (lbo unused).
+// M-major: [64 k][64 m elements] boxes, 8-k groups 1024 bytes apart, the next 64 m elements lbo bytes further.
+__device__ __forceinline__ uint64_t pf_smem_desc(uint32_t addr, uint32_t lbo) {
   uint64_t d = 0;
-  d |= static_cast<uint64_t>((pf_smem(tile) & 0x3ffffu) >> 4);  // start address
-  d |= static_cast<uint64_t>(1) << 16;                           // leading byte offset (unused with swizzle)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                   // stride byte offset
-  d |= static_cast<uint64_t>(1) << 46;                           // descriptor version (Blackwell)
-  d |= static_cast<uint64_t>(2) << 61;                           // SWIZZLE_128B
+  d |= static_cast<uint64_t>((addr & 0x3ffffu) >> 4);   // start address
+  d |= static_cast<uint64_t>(lbo >> 4) << 16;            // leading byte offset
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;           // stride byte offset
+  d |= static_cast<uint64_t>(1) << 46;                   // descriptor version (Blackwell)
+  d |= static_cast<uint64_t>(2) << 61;                   // SWIZZLE_128B
   return d;
 }
 __device__ __forceinline__ void pf_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       :
-      : "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Arrives on the barrier at this offset in both CTAs once the MMAs issued so far are done.
 __device__ __forceinline__ void pf_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(pf_smem(bar)) : "memory");
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(pf_smem(bar)),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
 }
 __device__ __forceinline__ void pf_ld32(uint32_t taddr, float* v) {
   uint32_t r[32];
@@ -130,218 +157,322 @@ __device__ __forceinline__ void pf_ld32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Store n (<= 32) consecutive values of one row as T; 16-byte vectors when the address allows.
-template <typename T>
-__device__ __forceinline__ void pf_store_row(T* dst, const float* v, int n) {
-  if (n == 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      __align__(16) T tmp[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) tmp[e] = DT<T>::from_f(v[q * 8 + e]);
-      *reinterpret_cast<uint4*>(dst + q * 8) = *reinterpret_cast<const uint4*>(tmp);
+// Boxes of 64, 32, 16 and 8 rows of the same weights.
+struct PfWeightMaps {
+  CUtensorMap m[4];
+};
+
+// Box of at least `rows` rows: 1 + its index in PfWeightMaps, 0 for none.  A box may fetch rows beyond the CTA's share
+// (its neighbour's, on their way through the L2 anyway); their products land in accumulator lanes that nobody reads.
+__device__ __forceinline__ int pf_box(int rows) { return rows > 32 ? 1 : rows > 16 ? 2 : rows > 8 ? 3 : rows > 0 ? 4 : 0; }
+
+// One tile of a pair's walk.
+struct PfTile {
+  int m0, m_rows0, m_rows1;  // first M row of the tile (neuron / column); neurons of the even and the odd CTA
+  int tok0;                  // first token
+  int zi, kb_lo, nkb;        // contraction split and its k-blocks
+};
+
+// How the tiles of a launch are laid out.  Host-visible sizes give the grid; the device-side K decides here.
+struct PfPlan {
+  int w_tiles, tw, cover, tiles;  // M tiles, M rows per tile, M rows to cover, tiles in all
+  int nkb_all, splits, tok_tiles, n_tok;
+};
+
+template <int MODE>
+__device__ __forceinline__ PfPlan pf_plan(const PfArgs& p, int k_valid) {
+  PfPlan q;
+  q.splits = MODE == 1 ? max(1, p.splits) : 1;
+  q.tok_tiles = p.tok_tiles;
+  q.n_tok = p.n_tok;
+  if (MODE == 0) {
+    // with a device-side K the rows up to the end of its k-block are GEMM 2's operand too: zeros
+    q.cover = p.k_dev ? min(p.N, (k_valid + PF_BK - 1) / PF_BK * PF_BK) : p.N;
+    q.w_tiles = (q.cover + PF_TW - 1) / PF_TW;
+    q.tw = PF_TW;
+    if (p.even && q.cover > 0) {
+      // One token tile: every weight row is read once and the launch is bound by HBM, so all pairs
+      // take the same number of neurons (in 8s) instead of full tiles and a nearly empty last wave.
+      const int want = (q.w_tiles + p.pairs - 1) / p.pairs * p.pairs;
+      q.tw = max(16, ((q.cover + want - 1) / want + 7) / 8 * 8);
+      q.w_tiles = (q.cover + q.tw - 1) / q.tw;
     }
+    q.nkb_all = (p.Kd + PF_BK - 1) / PF_BK;
   } else {
-    for (int e = 0; e < n; ++e) dst[e] = DT<T>::from_f(v[e]);
+    q.cover = p.N;
+    q.tw = PF_HW;
+    q.w_tiles = (p.N + PF_HW - 1) / PF_HW;
+    q.nkb_all = ((p.k_dev ? min(p.Kd, k_valid) : p.Kd) + PF_BK - 1) / PF_BK;
   }
+  q.tiles = q.w_tiles * q.tok_tiles * q.splits;
+  return q;
 }
 
-// Dynamic shared memory (1024-byte aligned): stages x (A tile | B tile [| second B tile]);
-// then full[stages], empty[stages], accum barrier, TMEM base address.
-// DK: the device-side row count and the split of the contraction are compiled in (layer step on the
-// packed cache); the plain operator call uses the variant without them.
-template <typename T, int MODE, int MH, bool DK>
-__global__ void __launch_bounds__(PF_THREADS, 1)
-k_umma_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PfArgs p) {
+template <int MODE>
+__device__ __forceinline__ PfTile pf_tile(const PfPlan& q, int it) {
+  PfTile t;
+  const int per_split = q.w_tiles * q.tok_tiles;
+  t.zi = it / per_split;
+  const int i = it - t.zi * per_split;
+  // PF_GROUP token tiles walk the weights together: what is in flight shares both operands in the L2
+  const int g = i / (PF_GROUP * q.w_tiles);
+  const int gn = min(PF_GROUP, q.tok_tiles - g * PF_GROUP);
+  const int rem = i - g * PF_GROUP * q.w_tiles;
+  const int w = rem / gn;
+  t.tok0 = (g * PF_GROUP + rem - w * gn) * q.n_tok;
+  t.m0 = w * q.tw;
+  if (MODE == 0) {
+    const int n8 = (min(q.tw, q.cover - t.m0) + 7) / 8;  // groups of 8 neurons
+    t.m_rows0 = (n8 + 1) / 2 * 8;
+    t.m_rows1 = n8 / 2 * 8;
+  } else {
+    t.m_rows0 = t.m_rows1 = 128;
+  }
+  t.kb_lo = static_cast<int>(static_cast<long long>(q.nkb_all) * t.zi / q.splits);
+  t.nkb = static_cast<int>(static_cast<long long>(q.nkb_all) * (t.zi + 1) / q.splits) - t.kb_lo;
+  return t;
+}
+
+// tmA[i]: weights, box 64 k x (64 >> i) rows (MODE 0) / [0] only, 64 columns x 64 k rows (MODE 1); tmB: tokens, box 64 x n_tok/2.  Dynamic shared memory (1024-byte aligned): stages x (A tile | token tile),
+// exchange buffers of the epilogue, then full[S], empty[S], acc_full[2], acc_empty[2], TMEM base address.
+template <typename T, int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PF_THREADS, 1)
+k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CUtensorMap tmB, const PfArgs p) {
   extern __shared__ unsigned char pf_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(pf_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  constexpr uint32_t STAGE_BYTES = (MH + 2) * PF_TILE_BYTES;   // MH A tiles, 2 B tiles
-  constexpr uint32_t TMEM_COLS = MH * 2 * PF_BN;               // accumulator (mh, nt) at column (2*mh + nt) * 128
   const int S = p.stages;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(S) * STAGE_BYTES);
+  const uint32_t b_bytes = static_cast<uint32_t>(p.n_tok / 2) * (PF_BK * 2);
+  const uint32_t stage_bytes = PF_A_BYTES + b_bytes;  // n_tok/2 is a multiple of 16: 1024-byte aligned stages
+  float* xch = reinterpret_cast<float*>(smem + static_cast<size_t>(S) * stage_bytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(xch) + PF_XCH_BYTES);
   uint64_t* empty = full + S;
-  uint64_t* accum = empty + S;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+  uint64_t* acc_full = empty + S;
+  uint64_t* acc_empty = acc_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // MODE 0: row tiles vary fastest, so CTAs in flight share weight tiles and x (which fits L2)
-  // is the re-read operand; MODE 1: column tiles vary fastest (the transposed down weight fits L2)
-  const int n_idx = MODE == 0 ? blockIdx.y : blockIdx.x, m_idx = MODE == 0 ? blockIdx.x : blockIdx.y;
-  const int n0 = n_idx * (MODE == 0 ? PF_BN : 2 * PF_BN), m0 = m_idx * (MH * PF_BM);
-  const int k_valid = (DK && p.k_dev) ? *p.k_dev : 0x7fffffff;
-  const int k_round = k_valid > 0x7fffff00 ? k_valid : (k_valid + PF_BK - 1) / PF_BK * PF_BK;
-  if (DK && MODE == 0 && n0 >= k_round) return;  // nothing downstream reads these columns (uniform for the CTA)
-  const int nkb_all = (min(p.Kd, MODE == 1 ? k_valid : p.Kd) + PF_BK - 1) / PF_BK;
-  // this CTA's k-blocks [kb_lo, kb_lo + nkb)
-  const int nz = DK ? static_cast<int>(gridDim.z) : 1, zi = DK ? static_cast<int>(blockIdx.z) : 0;
-  const int kb_lo = (nkb_all * zi) / nz;
-  const int nkb = (nkb_all * (zi + 1)) / nz - kb_lo;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       pf_mbar_init(&full[s], 1);
       pf_mbar_init(&empty[s], 1);
     }
-    pf_mbar_init(accum, 1);
+    for (int b = 0; b < 2; ++b) {
+      pf_mbar_init(&acc_full[b], 1);
+      pf_mbar_init(&acc_empty[b], 8);  // four epilogue warps of either CTA
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {  // tensor memory: one warp allocates, the same warp frees
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pf_smem(tmem_slot)), "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (warp == 1) {  // tensor memory: this warp of both CTAs allocates, the same warps free
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pf_smem(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  const uint32_t full0 = pf_mapa(full, 0);  // the even CTA's barriers
+  const int k_valid = p.k_dev ? min(*p.k_dev, MODE == 0 ? p.N : p.Kd) : (MODE == 0 ? p.N : p.Kd);
+  const PfPlan plan = pf_plan<MODE>(p, k_valid);
   bool timed_out = false;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == 0 || warp >= 6) {
+    // ------------------------------------------------------------------ TMA producers
     if (lane == 0) {
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % S;
-        if (kb >= S && !pf_wait(&empty[s], ((kb / S) - 1) & 1)) timed_out = true;
-        unsigned char* st = smem + static_cast<size_t>(s) * STAGE_BYTES;
-        pf_expect_tx(&full[s], STAGE_BYTES);
-#pragma unroll
-        for (int mh = 0; mh < MH; ++mh)
-          pf_tma_2d(st + mh * PF_TILE_BYTES, &tmA, (kb_lo + kb) * PF_BK, m0 + mh * PF_BM, &full[s]);
-        pf_tma_2d(st + MH * PF_TILE_BYTES, &tmB, (kb_lo + kb) * PF_BK, n0, &full[s]);
-        pf_tma_2d(st + (MH + 1) * PF_TILE_BYTES, &tmB, (kb_lo + kb) * PF_BK, MODE == 0 ? p.up_off + n0 : n0 + PF_BN, &full[s]);
+      const int part = warp == 0 ? 0 : warp - 5;  // 0, 1: the halves of the A tile, 2: tokens
+      int s = 0;
+      uint32_t phase = 1;  // the first round finds every stage free
+      for (int it = pair; it < plan.tiles && !timed_out; it += npairs) {
+        const PfTile t = pf_tile<MODE>(plan, it);
+        const int box0 = pf_box(t.m_rows0), box1 = pf_box(t.m_rows1);
+        const uint32_t bytes = (MODE == 0 ? ((box0 ? 64u >> (box0 - 1) : 0u) + (box1 ? 64u >> (box1 - 1) : 0u)) * (2 * PF_BK * 2) : 2 * PF_A_BYTES) + 2 * b_bytes;
+        const int box = rank ? box1 : box0;
+        const int m0 = MODE == 0 ? t.m0 + (rank ? t.m_rows0 : 0) + (part == 1 ? p.N : 0)
+                                 : t.m0 + static_cast<int>(rank) * 128 + part * 64;
+        const int tok = t.tok0 + static_cast<int>(rank) * (p.n_tok / 2);
+        const CUtensorMap* map = part == 2 ? &tmB : &tmA.m[MODE == 0 && box > 1 ? box - 1 : 0];
+        const bool issue = part == 2 || MODE == 1 || box > 0;
+        int k = t.kb_lo * PF_BK;
+        for (int kb = 0; kb < t.nkb; ++kb, k += PF_BK) {
+          if (!pf_wait(&empty[s], phase)) {
+            timed_out = true;
+            break;
+          }
+          unsigned char* dst = smem + static_cast<size_t>(s) * stage_bytes + (part == 2 ? PF_A_BYTES : part * 8192u);
+          if (rank == 0 && part == 0) pf_expect_tx(&full[s], bytes);
+          if (issue) {
+            if (part == 2) pf_tma_2d(dst, map, k, tok, full0 + s * 8);
+            else if (MODE == 0) pf_tma_2d(dst, map, k, m0, full0 + s * 8);
+            else pf_tma_2d(dst, map, m0, k, full0 + s * 8);
+          }
+          if (++s == S) {
+            s = 0;
+            phase ^= 1;
+          }
+        }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      // instruction descriptor: D = f32, A/B = f16 or bf16, both K-major, N = 128, M = 128
-      const uint32_t fmt = sizeof(T) == 2 && DT<T>::id == STX_BF16 ? 1u : 0u;
-      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(PF_BN >> 3) << 17) |
-                             (static_cast<uint32_t>(PF_BM >> 4) << 24);
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % S;
-        if (!pf_wait(&full[s], (kb / S) & 1)) timed_out = true;
+    // ------------------------------------------------------------------ MMA issuer (even CTA)
+    if (rank == 0 && lane == 0) {
+      // instruction descriptor: D = f32, A/B = f16 or bf16, A M-major in MODE 1, M = 256
+      const uint32_t fmt = DT<T>::id == STX_BF16 ? 1u : 0u;
+      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((MODE == 1 ? 1u : 0u) << 15) |
+                             (static_cast<uint32_t>(p.n_tok >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
+      constexpr uint32_t A_STEP = MODE == 0 ? 32 : 2048;  // bytes of 16 k elements inside the A tile
+      int s = 0, na = 0;
+      uint32_t phase = 0;
+      for (int it = pair; it < plan.tiles && !timed_out; it += npairs) {
+        const PfTile t = pf_tile<MODE>(plan, it);
+        if (t.nkb == 0) continue;
+        const int buf = na & 1;
+        if (na >= 2 && !pf_wait(&acc_empty[buf], ((na >> 1) - 1) & 1)) {
+          timed_out = true;
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned char* st = smem + static_cast<size_t>(s) * STAGE_BYTES;
-        const uint64_t db0 = pf_smem_desc(st + MH * PF_TILE_BYTES), db1 = pf_smem_desc(st + (MH + 1) * PF_TILE_BYTES);
+        for (int kb = 0; kb < t.nkb; ++kb) {
+          if (!pf_wait(&full[s], phase)) {
+            timed_out = true;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t st = pf_smem(smem + static_cast<size_t>(s) * stage_bytes);
+          const uint64_t da = pf_smem_desc(st, MODE == 0 ? 16 : 8192), db = pf_smem_desc(st + PF_A_BYTES, 16);
 #pragma unroll
-        for (int kk = 0; kk < PF_BK / 16; ++kk) {
-          const uint32_t acc = (kb | kk) != 0;
-          const uint64_t adv = static_cast<uint64_t>(kk * 32 >> 4);  // 16 elements = 32 bytes along k
-#pragma unroll
-          for (int mh = 0; mh < MH; ++mh) {
-            const uint64_t da = pf_smem_desc(st + mh * PF_TILE_BYTES) + adv;
-            pf_mma(tmem_base + (2 * mh) * PF_BN, da, db0 + adv, idesc, acc);
-            pf_mma(tmem_base + (2 * mh + 1) * PF_BN, da, db1 + adv, idesc, acc);
+          for (int kk = 0; kk < PF_BK / 16; ++kk)
+            pf_mma(tmem_base + buf * PF_MAX_N, da + (kk * A_STEP >> 4), db + (kk * 32 >> 4), idesc, (kb | kk) != 0);
+          pf_commit(&empty[s]);
+          if (++s == S) {
+            s = 0;
+            phase ^= 1;
           }
         }
-        pf_commit(&empty[s]);  // arrives when the MMAs that read this stage are done
+        if (timed_out) break;
+        pf_commit(&acc_full[buf]);
+        ++na;
       }
-      pf_commit(accum);
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps 2..5
-    const int lg = warp & 3;                    // TMEM lane group this warp may read
-    if (!pf_wait(accum, 0)) timed_out = true;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int lg = warp & 3;  // TMEM lane group this warp may read
     T* out = static_cast<T*>(p.a_out);
     T* comb = static_cast<T*>(p.combined);
-#pragma unroll 1
-    for (int mh = 0; mh < MH; ++mh) {
-      const int row = m0 + mh * PF_BM + lg * 32 + lane;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + (2 * mh) * PF_BN;
+    const uint32_t acc_empty0[2] = {pf_mapa(&acc_empty[0], 0), pf_mapa(&acc_empty[1], 0)};
+    int na = 0;
+    for (int it = pair; it < plan.tiles && !timed_out; it += npairs) {
+      const PfTile t = pf_tile<MODE>(plan, it);
+      const int buf = na & 1;
+      const int ntok = min(p.n_tok, p.M - t.tok0);
+      if (t.nkb > 0) {
+        timed_out = __any_sync(0xffffffffu, !pf_wait(&acc_full[buf], (na >> 1) & 1));
+        if (MODE == 0) {  // the two warps of a pair leave the loop together
+          int dead = timed_out;
+          asm volatile(
+              "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\t"
+              "barrier.cta.red.or.pred b, %2, 64, a;\n\tselp.s32 %0, 1, 0, b;\n\t}"
+              : "=r"(dead)
+              : "r"(dead), "r"(1 + (lg & 1))
+              : "memory");
+          timed_out = dead != 0;
+        }
+        if (timed_out) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + buf * PF_MAX_N;
       if (MODE == 0) {
+        const int nl = (lg & 1) * 32 + lane;  // neuron inside the CTA's share
+        const int j = t.m0 + (rank ? t.m_rows0 : 0) + nl;
+        const bool mine = nl < (rank ? t.m_rows1 : t.m_rows0) && j < plan.cover;
+        const bool is_up = lg >= 2;
+        float* xp = xch + (lg & 1) * 2048;
+        // gate warps finish tokens 0..15 of a chunk, up warps tokens 16..31: each hands the other half over
 #pragma unroll 1
-        for (int c = 0; c < PF_BN; c += 32) {
-          float g[32], u[32];
-          pf_ld32(taddr + c, g);
-          pf_ld32(taddr + PF_BN + c, u);
-          const int col = n0 + c;
-          const int n = min(32, p.N - col);
-          if (DK && p.part) {  // split contraction: raw partial sums, the activation follows the sum
-            if (row < p.M && n > 0) {
-              float* dst = p.part + (static_cast<size_t>(zi) * p.M + row) * (2 * static_cast<size_t>(p.ld_part)) + col;
-              for (int e = 0; e < n; ++e) {
-                dst[e] = nkb > 0 ? g[e] : 0.f;
-                dst[p.ld_part + e] = nkb > 0 ? u[e] : 0.f;
-              }
-            }
-            continue;
-          }
+        for (int c = 0; c < p.n_tok; c += 32) {
+          if (c >= ntok) break;
+          float v[32];
+          pf_ld32(taddr + c, v);
+          float* xb = xp + ((c >> 5) & 1) * 1024;
+          float* give = xb + (is_up ? 512 : 0);
+          const float* take = xb + (is_up ? 0 : 512);
+          if (is_up) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) g[e] = (!DK || col + e < k_valid) ? apply_act(p.act, g[e]) * u[e] : 0.f;
-          if (row < p.M && n > 0) {
-            if (out) pf_store_row<T>(out + static_cast<size_t>(row) * p.ld_out + col, g, n);
-            if (comb) {
-              pf_store_row<T>(comb + static_cast<size_t>(row) * (2 * p.N) + col, g, n);
-              pf_store_row<T>(comb + static_cast<size_t>(row) * (2 * p.N) + p.N + col, u, n);
+            for (int e = 0; e < 16; ++e) give[e * 32 + lane] = v[e];
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) give[e * 32 + lane] = v[16 + e];
+          }
+          asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + (lg & 1)) : "memory");
+          if (mine) {
+            const int tb = c + (is_up ? 16 : 0);
+            const size_t row0 = static_cast<size_t>(t.tok0 + tb);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float other = take[e * 32 + lane];
+              const float g = is_up ? other : v[e], u = is_up ? v[16 + e] : other;
+              if (tb + e < ntok) {
+                const T a = DT<T>::from_f(j < k_valid ? apply_act(p.act, g) * u : 0.f);
+                if (out) out[(row0 + e) * p.ld_out + j] = a;
+                if (comb) {
+                  T* cr = comb + (row0 + e) * (2 * static_cast<size_t>(p.N)) + j;
+                  cr[0] = a;
+                  cr[p.N] = DT<T>::from_f(u);
+                }
+              }
             }
           }
         }
       } else {
+        const int col = t.m0 + static_cast<int>(rank) * 128 + lg * 32 + lane;
 #pragma unroll 1
-        for (int c = 0; c < 2 * PF_BN; c += 32) {
-          float g[32];
-          pf_ld32(taddr + c, g);
-          if (DK && nkb == 0) {  // empty contraction: the accumulator was never written
+        for (int c = 0; c < p.n_tok; c += 32) {
+          if (c >= ntok) break;
+          float v[32];
+          if (t.nkb > 0) {
+            pf_ld32(taddr + c, v);
+          } else {  // empty contraction: the accumulator was never written
 #pragma unroll
-            for (int e = 0; e < 32; ++e) g[e] = 0.f;
+            for (int e = 0; e < 32; ++e) v[e] = 0.f;
           }
-          const int col = n0 + c;
-          const int n = min(32, p.N - col);
-          if (row < p.M && n > 0) {
-            if (DK && p.part) {
-              float* dst = p.part + (static_cast<size_t>(zi) * p.M + row) * p.ld_out + col;
-              for (int e = 0; e < n; ++e) dst[e] = g[e];
+          if (col < p.N) {
+            const size_t row0 = static_cast<size_t>(t.tok0 + c);
+            if (p.part) {
+              float* dst = p.part + (static_cast<size_t>(t.zi) * p.M + row0) * p.ld_out + col;
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (c + e < ntok) dst[static_cast<size_t>(e) * p.ld_out] = v[e];
             } else {
-              pf_store_row<T>(out + static_cast<size_t>(row) * p.ld_out + col, g, n);
+              T* dst = out + row0 * p.ld_out + col;
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (c + e < ntok) dst[static_cast<size_t>(e) * p.ld_out] = DT<T>::from_f(v[e]);
             }
           }
         }
+      }
+      if (t.nkb > 0) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) pf_arrive_cluster(acc_empty0[buf]);
+        ++na;
       }
     }
   }
   if (timed_out && p.status && lane == 0) atomicOr(p.status, DEV_TIMEOUT);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  // neither CTA leaves (or frees tensor memory) while the other's copies and commits may still reach its barriers
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
-  }
-}
-
-// [R, C] -> [C, ldo] (ldo >= R): packed down rows to the K-major B operand of GEMM 2.  64 x 64
-// tiles of 16-bit elements, 16-byte global loads and stores on both sides; requires C % 8 == 0 and
-// ldo % 8 == 0.  Rows >= R read as zero.  r_dev (optional): device-side row count, rows beyond its
-// k-block are never reached by the contraction and are skipped.
-__global__ void __launch_bounds__(256) k_pf_transpose(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int R, int C,
-                                                      int ldo, const int* __restrict__ r_dev) {
-  // the tile is stored transposed ([column][row], rows of 66 elements: the 8 column groups a warp
-  // scatters into land in 4 different bank quarters) and read back with aligned 32-bit loads
-  __shared__ __align__(16) uint16_t tile[64][66];
-  const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
-  if (r_dev && r0 >= (*r_dev + PF_BK - 1) / PF_BK * PF_BK) return;
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {  // 64 rows x 8 chunks of 8 elements
-    const int idx = t + 256 * k, rr = idx >> 3, cc = (idx & 7) * 8;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r0 + rr < R && c0 + cc < C) v = *reinterpret_cast<const uint4*>(in + static_cast<size_t>(r0 + rr) * C + c0 + cc);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      tile[cc + 2 * e][rr] = static_cast<uint16_t>(w[e] & 0xffffu);
-      tile[cc + 2 * e + 1][rr] = static_cast<uint16_t>(w[e] >> 16);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {  // 64 output rows (columns of the input tile) x 8 chunks of 8 input rows
-    const int idx = t + 256 * k, cc = idx >> 3, rr = (idx & 7) * 8;
-    if (c0 + cc < C && r0 + rr < ldo) {
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(&tile[cc][rr]);  // 132-byte rows: 4-byte aligned
-      const uint4 v = make_uint4(src[0], src[1], src[2], src[3]);
-      *reinterpret_cast<uint4*>(out + static_cast<size_t>(c0 + cc) * ldo + r0 + rr) = v;
-    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
 }
 
@@ -362,103 +493,87 @@ static PFN_encodeTiled encode_fn() {
   return fn;
 }
 
-// 2-D K-major operand [rows, kd] with row stride ld (elements); box 64 x 128, 128-byte swizzle.
-static int make_map(CUtensorMap* m, const void* base, int dtype, int64_t rows, int64_t kd, int64_t ld) {
+// 2-D operand [rows, cols] of 16-bit elements with row stride ld (elements), 128-byte swizzle.
+static int make_map(CUtensorMap* m, const void* base, int dtype, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
   PFN_encodeTiled enc = encode_fn();
   if (!enc) {
     set_error("prefill path: cuTensorMapEncodeTiled is not available from this driver");
     return STX_ERR_CUDA;
   }
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(kd), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-  const cuuint32_t box[2] = {PF_BK, PF_BM};
+  const cuuint32_t box[2] = {PF_BK, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(m, dtype == STX_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                          const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    set_error("prefill path: cuTensorMapEncodeTiled failed with %d (rows=%lld k=%lld ld=%lld)", static_cast<int>(r),
-              static_cast<long long>(rows), static_cast<long long>(kd), static_cast<long long>(ld));
+    set_error("prefill path: cuTensorMapEncodeTiled failed with %d (rows=%lld cols=%lld ld=%lld)", static_cast<int>(r),
+              static_cast<long long>(rows), static_cast<long long>(cols), static_cast<long long>(ld));
     return STX_ERR_CUDA;
   }
   return STX_OK;
 }
 
-template <typename T, int MODE, int MH, bool DK>
-static int launch_umma_dk(const CUtensorMap& a, const CUtensorMap& b, PfArgs p, cudaStream_t s) {
-  constexpr uint32_t stage_bytes = (MH + 2) * PF_TILE_BYTES;
-  p.stages = MH == 2 ? 3 : 4;
-  const size_t smem = 1024 + static_cast<size_t>(p.stages) * stage_bytes + (2 * p.stages + 1) * sizeof(uint64_t) + 16;
+static int sm_pairs() { return std::max(1, num_sms() / 2); }
+
+template <typename T, int MODE>
+static int launch_pair(const PfWeightMaps& a, const CUtensorMap& b, PfArgs p, int tiles, cudaStream_t s) {
   static bool attr_set[64] = {};
   int dev = 0;
-  cudaGetDevice(&dev);
+  STX_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    STX_CUDA(cudaFuncSetAttribute(k_umma_gemm<T, MODE, MH, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    STX_CUDA(cudaFuncSetAttribute(k_pair_gemm<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     attr_set[dev] = true;
   }
-  const int bn = MODE == 0 ? PF_BN : 2 * PF_BN, bm = MH * PF_BM;
-  dim3 grid((p.N + bn - 1) / bn, (p.M + bm - 1) / bm, static_cast<unsigned>(std::max(1, p.stages_z)));
-  if (MODE == 0) grid = dim3(grid.y, grid.x, grid.z);
-  k_umma_gemm<T, MODE, MH, DK><<<grid, PF_THREADS, smem, s>>>(a, b, p);
-  STX_LAUNCH_CHECK("k_umma_gemm");
+  const uint32_t stage_bytes = PF_A_BYTES + static_cast<uint32_t>(p.n_tok / 2) * (PF_BK * 2);
+  const uint32_t fixed = 1024 + PF_XCH_BYTES + (2 * PF_MAX_STAGES + 4) * 8 + 16;
+  p.stages = static_cast<int>(std::min<uint32_t>(PF_MAX_STAGES, (PF_SMEM - fixed) / stage_bytes));
+  p.pairs = sm_pairs();
+  const size_t smem = fixed + static_cast<size_t>(p.stages) * stage_bytes;
+  const unsigned grid = 2u * static_cast<unsigned>(std::max(1, std::min(tiles, p.pairs)));
+  STX_CUDA(launch_pdl(k_pair_gemm<T, MODE>, dim3(grid), dim3(PF_THREADS), smem, s, a, b, p));
   return STX_OK;
 }
 
-template <typename T, int MODE, int MH>
-static int launch_umma_mh(const CUtensorMap& a, const CUtensorMap& b, const PfArgs& p, cudaStream_t s) {
-  return (p.k_dev || p.part) ? launch_umma_dk<T, MODE, MH, true>(a, b, p, s) : launch_umma_dk<T, MODE, MH, false>(a, b, p, s);
-}
-
-template <typename T, int MODE>
-static int launch_umma(const CUtensorMap& a, const CUtensorMap& b, const PfArgs& p, cudaStream_t s) {
-  // one row half for small row counts, two (a 256-row CTA tile) otherwise
-  return p.M > PF_BM ? launch_umma_mh<T, MODE, 2>(a, b, p, s) : launch_umma_mh<T, MODE, 1>(a, b, p, s);
-}
-
-// a[b][j] = act(sum_z gate_z[b][j]) * sum_z up_z[b][j] for j < K (zero up to the end of K's k-block),
-// z ascending: the tail of a GEMM 1 whose contraction was split.
-template <typename T>
-__global__ void __launch_bounds__(256) k_pf_act_sum(const float* __restrict__ part, int nz, int M, int N, int ldp,
-                                                    T* __restrict__ a_out, int ld_out, int act, const int* __restrict__ k_dev) {
-  const int k_valid = k_dev ? min(*k_dev, N) : N;
-  const int k_round = min(N, (k_valid + PF_BK - 1) / PF_BK * PF_BK);
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-  if (j >= k_round || b >= M) return;
-  float g = 0.f, u = 0.f;
-  for (int z = 0; z < nz; ++z) {
-    const float* src = part + (static_cast<size_t>(z) * M + b) * (2 * static_cast<size_t>(ldp)) + j;
-    g += __ldcg(src);
-    u += __ldcg(src + ldp);
+// Tokens of a tile and contraction splits of one launch, by an estimate of its time: a k-block of a
+// tile takes the pair 2 clocks per token of the tile on the tensor pipe, and 0.37 us for its 32 KB of
+// weights at an even share of HBM when no other token tile reads the same ones; whole waves of tiles
+// count.  Splits (partial sums in fp32, added by one more kernel) pay where the tiles are too few.
+struct PfShape {
+  int n_tok, tok_tiles, splits;
+};
+constexpr int64_t PF_SPLIT_ROWS = 2048;  // splits x tokens of the partial sums
+static PfShape pair_shape(int64_t B, int64_t m_tiles, int64_t nkb, int64_t H, bool may_split, bool even) {
+  PfShape best = {0, 0, 1};
+  double best_t = 1e30;
+  const int64_t t_min = (B + PF_MAX_N - 1) / PF_MAX_N;
+  for (int64_t tt = t_min; tt <= t_min + std::max<int64_t>(2, t_min / 4); ++tt) {
+    const int64_t n = ((B + tt - 1) / tt + 31) / 32 * 32;
+    const int64_t tiles_t = (B + n - 1) / n;
+    if (tiles_t > 1 && n < 96) break;
+    const double kb_us = std::max(0.37 / static_cast<double>(std::min<int64_t>(tiles_t, PF_GROUP)), 0.0011 * static_cast<double>(n));
+    for (int64_t z = 1; z <= (may_split ? 16 : 1); ++z) {
+      if (z > 1 && (z * B > PF_SPLIT_ROWS || z > nkb)) break;
+      const double tiles = static_cast<double>(m_tiles * tiles_t * z), pairs = sm_pairs();
+      const double waves = even && tiles_t == 1 ? tiles / pairs : static_cast<double>((m_tiles * tiles_t * z + sm_pairs() - 1) / sm_pairs());
+      double t = waves * static_cast<double>((nkb + z - 1) / z) * kb_us;
+      if (z > 1) t += 3.0 + 8.0 * static_cast<double>(z * B * H) / 5e6;
+      if (t < best_t * 0.999) {
+        best_t = t;
+        best = {static_cast<int>(n), static_cast<int>(tiles_t), static_cast<int>(z)};
+      }
+    }
   }
-  a_out[static_cast<size_t>(b) * ld_out + j] = DT<T>::from_f(j < k_valid ? apply_act(act, g) * u : 0.f);
-}
-
-// GEMM 1 has ceil(B/128..256) x I/128 output tiles: a shard of the intermediate dimension with few rows
-// leaves most SMs without one, so its contraction (over H) is split too.
-static int gemm1_splits(int64_t B, int64_t H, int64_t K) {
-  const int64_t bm = B > PF_BM ? 2 * PF_BM : PF_BM;
-  const int64_t tiles = ((B + bm - 1) / bm) * ((K + PF_BN - 1) / PF_BN);
-  if (tiles > num_sms()) return 1;
-  // round up: the tiles are counted for all K slots, but a cache is rarely full (tiles beyond the
-  // device-side K exit at once), so up to 2x the SM count of CTAs still runs as about one wave
-  return static_cast<int>(std::min<int64_t>({8, (num_sms() + tiles - 1) / tiles, std::max<int64_t>(1, H / (4 * PF_BK))}));
-}
-
-// GEMM 2 has only ceil(B/128..256) x H/256 output tiles; for few rows the contraction is split so
-// that about one CTA per SM streams the down weight.
-static int gemm2_splits(int64_t B, int64_t H) {
-  const int64_t tiles = ((B + (B > PF_BM ? 2 * PF_BM : PF_BM) - 1) / (B > PF_BM ? 2 * PF_BM : PF_BM)) * ((H + 2 * PF_BN - 1) / (2 * PF_BN));
-  if (tiles * 2 > num_sms()) return 1;
-  return static_cast<int>(std::min<int64_t>(16, std::max<int64_t>(1, num_sms() / tiles)));
+  return best;
 }
 
 size_t prefill_scratch_bytes(int64_t B, int64_t H, int64_t K) {
   const int64_t K8 = (K + 7) / 8 * 8;
-  const int z = gemm2_splits(B, H), z1 = gemm1_splits(B, H, K);
-  return align_up(static_cast<size_t>(B) * K8 * 2, 1024) + align_up(static_cast<size_t>(H) * K8 * 2, 1024) + 1024 +
-         (z > 1 ? align_up(static_cast<size_t>(z) * B * H * sizeof(float), 1024) : 0) +
-         (z1 > 1 ? align_up(static_cast<size_t>(z1) * B * 2 * K8 * sizeof(float), 1024) : 0);
+  // activations [B, K8], partial sums of a split GEMM 2 (at most 16 splits and PF_SPLIT_ROWS rows in all): grows with B
+  return 1024 + align_up(static_cast<size_t>(B) * K8 * 2, 1024) +
+         align_up(static_cast<size_t>(std::min<int64_t>(16 * B, PF_SPLIT_ROWS)) * H * sizeof(float), 1024);
 }
 
 // Implemented in stx_mlp_row.cu: out[i] = sum over g < G of partial[g][i], g ascending (n % 128 == 0).
@@ -467,6 +582,13 @@ int partial_sum(const float* partial, int G, int64_t n, void* out, int dtype, cu
 // Row blocks of STX_GEMM_MIN_ROWS and more (16-bit, gated) run as tensor-core GEMMs.
 bool prefill_wanted(int64_t B, int64_t H, int64_t K, int dtype, int has_gate) {
   return dtype != STX_F32 && has_gate && B >= STX_GEMM_MIN_ROWS && (H % 64) == 0 && K >= 64;
+}
+
+template <typename T>
+static int prefill_run(const PfWeightMaps& mw, const CUtensorMap& mx, const PfArgs& g1, int tiles1, const PfWeightMaps& md,
+                       const CUtensorMap& ma, const PfArgs& g2, int tiles2, cudaStream_t s) {
+  const int rc = launch_pair<T, 0>(mw, mx, g1, tiles1, s);
+  return rc != STX_OK ? rc : launch_pair<T, 1>(md, ma, g2, tiles2, s);
 }
 
 // x [B,H], concat [2K,H] (gate rows then up rows), down_packed [K,H]; scratch: prefill_scratch_bytes().
@@ -478,33 +600,32 @@ int prefill_forward(const void* x, int64_t B, int64_t H, const void* concat, con
   const int64_t K8 = (K + 7) / 8 * 8;
   const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 1023) & ~static_cast<uintptr_t>(1023);
   void* a_scr = reinterpret_cast<void*>(base);                                                   // [B, K8]
-  void* dt_scr = reinterpret_cast<void*>(base + align_up(static_cast<size_t>(B) * K8 * 2, 1024));  // [H, K8]
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(concat)) & 15) {
-    set_error("prefill path: x and concat_w must be 16-byte aligned");
+  float* part = reinterpret_cast<float*>(base + align_up(static_cast<size_t>(B) * K8 * 2, 1024));
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(concat) | reinterpret_cast<uintptr_t>(down_packed)) & 15) {
+    set_error("prefill path: x, concat_w and down_packed must be 16-byte aligned");
     return STX_ERR_INVALID_ARG;
   }
-  // down rows -> K-major [H, K8]
-  {
-    dim3 grid(static_cast<unsigned>((H + 63) / 64), static_cast<unsigned>((K + 63) / 64));
-    k_pf_transpose<<<grid, 256, 0, s>>>(static_cast<const uint16_t*>(down_packed), static_cast<uint16_t*>(dt_scr),
-                                                 static_cast<int>(K), static_cast<int>(H), static_cast<int>(K8), k_dev);
-    STX_LAUNCH_CHECK("k_pf_transpose");
-  }
-  // the activations are GEMM 2's A operand: read them straight from combined_buf[:, :K] when its
+  const int64_t w_tiles = (K + PF_TW - 1) / PF_TW, h_tiles = (H + PF_HW - 1) / PF_HW;
+  const PfShape s1 = pair_shape(B, w_tiles, (H + PF_BK - 1) / PF_BK, H, false, true);
+  const PfShape s2 = pair_shape(B, h_tiles, (K + PF_BK - 1) / PF_BK, H, (B * H) % 128 == 0, false);
+  // the activations are GEMM 2's token operand: read them straight from combined_buf[:, :K] when its
   // row stride is TMA-compatible (a multiple of 16 bytes), else from the scratch copy
   const bool a_in_combined = combined != nullptr && (K % 4) == 0 && (reinterpret_cast<uintptr_t>(combined) & 15) == 0;
-  CUtensorMap mx, mw, ma, md;
-  int rc = make_map(&mx, x, dtype, B, H, H);
-  if (rc == STX_OK) rc = make_map(&mw, concat, dtype, 2 * K, H, H);
-  if (rc == STX_OK) rc = a_in_combined ? make_map(&ma, combined, dtype, B, K, 2 * K) : make_map(&ma, a_scr, dtype, B, K, K8);
-  if (rc == STX_OK) rc = make_map(&md, dt_scr, dtype, H, K, K8);
+  CUtensorMap mx, ma;
+  PfWeightMaps mw, md = {};
+  int rc = make_map(&mx, x, dtype, B, H, H, s1.n_tok / 2);
+  for (int i = 0; i < 4 && rc == STX_OK; ++i) rc = make_map(&mw.m[i], concat, dtype, 2 * K, H, H, 64 >> i);
+  if (rc == STX_OK)
+    rc = a_in_combined ? make_map(&ma, combined, dtype, B, K, 2 * K, s2.n_tok / 2) : make_map(&ma, a_scr, dtype, B, K, K8, s2.n_tok / 2);
+  if (rc == STX_OK) rc = make_map(&md.m[0], down_packed, dtype, K, H, H, PF_BK);
   if (rc != STX_OK) return rc;
   PfArgs g1{};
   g1.M = static_cast<int>(B);
   g1.N = static_cast<int>(K);
   g1.Kd = static_cast<int>(H);
-  g1.up_off = static_cast<int>(K);
-  g1.stages = 4;
+  g1.n_tok = s1.n_tok;
+  g1.tok_tiles = s1.tok_tiles;
+  g1.even = s1.tok_tiles == 1;
   g1.a_out = a_in_combined ? nullptr : a_scr;
   g1.ld_out = static_cast<int>(K8);
   g1.combined = combined;
@@ -515,49 +636,21 @@ int prefill_forward(const void* x, int64_t B, int64_t H, const void* concat, con
   g2.M = static_cast<int>(B);
   g2.N = static_cast<int>(H);
   g2.Kd = static_cast<int>(K);
-  g2.stages = 6;
+  g2.n_tok = s2.n_tok;
+  g2.tok_tiles = s2.tok_tiles;
+  g2.splits = s2.splits;
   g2.a_out = out;
   g2.ld_out = static_cast<int>(H);
   g2.act = act;
   g2.status = status;
   g2.k_dev = k_dev;
-  const int z_sized = gemm2_splits(B, H);  // what prefill_scratch_bytes reserved
-  const int z = (B * H) % 128 == 0 ? z_sized : 1;
-  float* part = nullptr;
-  const uintptr_t part_base = base + align_up(static_cast<size_t>(B) * K8 * 2, 1024) + align_up(static_cast<size_t>(H) * K8 * 2, 1024);
-  if (z > 1) {
-    part = reinterpret_cast<float*>(part_base);
-    g2.part = part;
-    g2.stages_z = z;
-  }
-  // GEMM 1 split (only without combined_buf: the activation moves to k_pf_act_sum, which writes a alone)
-  const int z1 = combined == nullptr ? gemm1_splits(B, H, K) : 1;
-  float* part1 = nullptr;
-  if (z1 > 1) {
-    part1 = reinterpret_cast<float*>(part_base + (z_sized > 1 ? align_up(static_cast<size_t>(z_sized) * B * H * sizeof(float), 1024) : 0));
-    g1.part = part1;
-    g1.ld_part = static_cast<int>(K8);
-    g1.stages_z = z1;
-  }
-  const dim3 agrid(static_cast<unsigned>((K + 255) / 256), static_cast<unsigned>(B));
-  if (dtype == STX_F16) {
-    rc = launch_umma<__half, 0>(mx, mw, g1, s);
-    if (rc == STX_OK && part1) {
-      k_pf_act_sum<__half><<<agrid, 256, 0, s>>>(part1, z1, static_cast<int>(B), static_cast<int>(K), static_cast<int>(K8),
-                                                 static_cast<__half*>(a_scr), static_cast<int>(K8), act, k_dev);
-      STX_LAUNCH_CHECK("k_pf_act_sum");
-    }
-    if (rc == STX_OK) rc = launch_umma<__half, 1>(ma, md, g2, s);
-  } else {
-    rc = launch_umma<__nv_bfloat16, 0>(mx, mw, g1, s);
-    if (rc == STX_OK && part1) {
-      k_pf_act_sum<__nv_bfloat16><<<agrid, 256, 0, s>>>(part1, z1, static_cast<int>(B), static_cast<int>(K), static_cast<int>(K8),
-                                                        static_cast<__nv_bfloat16*>(a_scr), static_cast<int>(K8), act, k_dev);
-      STX_LAUNCH_CHECK("k_pf_act_sum");
-    }
-    if (rc == STX_OK) rc = launch_umma<__nv_bfloat16, 1>(ma, md, g2, s);
-  }
-  if (rc == STX_OK && part) rc = partial_sum(part, z, B * H, out, dtype, s);
+  if (s2.splits > 1) g2.part = part;
+  // evenly shared neurons fill all pairs even where full tiles would not
+  const int tiles1 = g1.even ? sm_pairs() : static_cast<int>(w_tiles * s1.tok_tiles);
+  const int tiles2 = static_cast<int>(h_tiles * s2.tok_tiles * s2.splits);
+  rc = dtype == STX_F16 ? prefill_run<__half>(mw, mx, g1, tiles1, md, ma, g2, tiles2, s)
+                        : prefill_run<__nv_bfloat16>(mw, mx, g1, tiles1, md, ma, g2, tiles2, s);
+  if (rc == STX_OK && g2.part) rc = partial_sum(part, s2.splits, B * H, out, dtype, s);
   return rc;
 }
 
