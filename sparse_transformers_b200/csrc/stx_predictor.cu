@@ -79,6 +79,96 @@ k_pred_t(const T* __restrict__ x, const T* __restrict__ A, float* __restrict__ t
   }
 }
 
+// Sum of v[0..N) over the warp, each in the butterfly order of warp_sum_xor (the same bits: a + b == b + a), N a
+// power of two up to 32.  A stage halves the number of values a lane keeps: it hands over the half that its
+// partner keeps, so N values cost about N shuffles and not 5 N.  The lanes l with l >> (5 - log2 N) == j end with
+// value j (all of them with its sum).
+template <int N>
+__device__ __forceinline__ float warp_sum_xor_many(float (&v)[N], int lane) {
+  int n = N;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    if (n > 1) {
+      const bool hi = (lane & off) != 0;
+#pragma unroll
+      for (int j = 0; j < N / 2; ++j) {
+        if (j < n / 2) {
+          const float give = hi ? v[j] : v[j + n / 2];
+          const float keep = hi ? v[j + n / 2] : v[j];
+          v[j] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+      }
+      n /= 2;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    }
+  }
+  return v[0];
+}
+
+// t of row blocks: a block owns KT predictor rows x RT batch rows, thread u the chunks u, u + NT, ... of all of them,
+// so a loaded chunk of x serves KT sums and a chunk of A serves RT (k_pred_t reads x once per predictor row: 67 MB
+// through the L2 at 64 rows x 4096 x 128 and 8.6 GB at 8192 rows).  Arithmetic order of k_pred_t.
+// skip_words / n_skip (optional): the union built by earlier row chunks; once all I bits are set, no score of this
+// chunk can change it and the block returns.
+template <typename T, int KT, int RT, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+k_pred_t_rows(const T* __restrict__ x, const T* __restrict__ A, float* __restrict__ t_out, int B, int H, int r,
+              uint32_t* __restrict__ zero_words, int n_zero, const uint32_t* __restrict__ skip_words, int I) {
+  constexpr int V = DT<T>::V, NV = KT * RT;
+  __shared__ float s_ws[NV][33];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+  const int k0 = blockIdx.x * KT;
+  const int nchunk = H / V;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (skip_words) {
+    bool full = true;
+    for (int w = tid; w < (I + 31) / 32; w += blockDim.x) {
+      const uint32_t want = w * 32 + 32 <= I ? 0xffffffffu : (1u << (I & 31)) - 1u;
+      full = full && (__ldcg(skip_words + w) & want) == want;
+    }
+    if (__syncthreads_and(full)) return;
+  }
+  if (zero_words && blockIdx.y == 0)
+    for (int w = blockIdx.x * blockDim.x + tid; w < n_zero; w += gridDim.x * blockDim.x) zero_words[w] = 0u;
+  for (int b0 = blockIdx.y * RT; b0 < B; b0 += gridDim.y * RT) {
+    float acc[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) acc[j] = 0.f;
+    for (int c = tid; c < nchunk; c += blockDim.x) {
+      // rows beyond the edges repeat the last one: their sums are not stored
+      uint4 xr[RT], ar[KT];
+#pragma unroll
+      for (int k = 0; k < KT; ++k) ar[k] = ld_cached16(A + static_cast<size_t>(min(k0 + k, r - 1)) * H + c * V);
+#pragma unroll
+      for (int b = 0; b < RT; ++b) xr[b] = ld_cached16(x + static_cast<size_t>(min(b0 + b, B - 1)) * H + c * V);
+      float wa[KT][V];
+#pragma unroll
+      for (int k = 0; k < KT; ++k) Unpack<T>::run(ar[k], wa[k]);
+#pragma unroll
+      for (int b = 0; b < RT; ++b) {
+        float xv[V];
+        Unpack<T>::run(xr[b], xv);
+#pragma unroll
+        for (int k = 0; k < KT; ++k)
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[b * KT + k] = fmaf(xv[v], wa[k][v], acc[b * KT + k]);
+      }
+    }
+    constexpr int LPV = 32 / NV;  // lanes that end with the same value
+    const float s = warp_sum_xor_many<NV>(acc, lane);
+    if (lane % LPV == 0) s_ws[lane / LPV][wid] = s;
+    __syncthreads();
+    for (int j = wid; j < NV; j += nw) {
+      const float sum = warp_sum_xor(lane < nw ? s_ws[j][lane] : 0.f);
+      const int b = b0 + j / KT, k = k0 + j % KT;
+      if (lane == 0 && b < B && k < r) t_out[static_cast<size_t>(b) * r + k] = DT<T>::round_f(sum);
+    }
+    __syncthreads();
+  }
+}
+
 // One block (256 threads) per (mask word, group of PRED_BT batch rows): 8 lanes cooperate on one
 // neuron, 32 neurons per block.  Dynamic shared memory: the group's rows of t, fp32.  With more
 // than one group the blocks OR their words into `bits` (zeroed by the launcher): the union over
@@ -247,15 +337,30 @@ constexpr int PSM_LIST = 64;      // scores of a warp that wait for their evalua
 // fragment loads of eight rows then fall into different banks), Bpad = B rounded up to 8, rows >= B zero.
 template <typename T>
 __global__ void __launch_bounds__(PSM_WARPS * 32)
-k_pred_scores_mma(const float* __restrict__ t, const T* __restrict__ Bm, uint32_t* __restrict__ bits, int B, int r, int I, float tau) {
+k_pred_scores_mma(const float* __restrict__ t_all, const T* __restrict__ Bm, uint32_t* __restrict__ bits, int B_all, int row_tile, int r,
+                  int I, float tau, int merge) {
   extern __shared__ __align__(16) unsigned char psm_raw[];
   T* t_s = reinterpret_cast<T*>(psm_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, tq = lane & 3;
+  const int row0 = blockIdx.y * row_tile;
+  const int B = min(row_tile, B_all - row0);
+  const float* t = t_all + static_cast<size_t>(row0) * r;
   const int Bpad = (B + 7) & ~7, ts = r + 8, nspan = r >> 5;
   const int W = (I + 31) >> 5;
   const int w = blockIdx.x * PSM_WARPS + warp;
   const int i0 = w * 32;
+  const uint32_t word_full = i0 + 32 <= I ? 0xffffffffu : (1u << (I & 31)) - 1u;
+  if (merge) {
+    // The mask is the union over all rows: a word that other rows have filled already stays what it is, and a block
+    // whose words are all full has nothing to add.  (What is read here may be a moment old: bits are only ever set.)
+    pdl_wait();
+    const bool full = w >= W || (__ldcg(bits + w) & word_full) == word_full;
+    if (__syncthreads_and(full)) {
+      pdl_launch_dependents();
+      return;
+    }
+  }
 
   // weights first (they do not depend on the previous kernel): the chunks of this thread's four neurons
   uint4 alo[2][PSM_MAX_SPANS], ahi[2][PSM_MAX_SPANS];
@@ -413,20 +518,54 @@ k_pred_scores_mma(const float* __restrict__ t, const T* __restrict__ Bm, uint32_
     }
   }
   flush();
-  if (lane == 0) bits[w] = word;
+  if (lane == 0) {
+    if (!merge) bits[w] = word;
+    else if (word) atomicOr(&bits[w], word);
+  }
 }
+
+// Rows of one block of k_pred_scores_mma: t of that many rows (in the model dtype) stays within 48 KB of shared memory.
+constexpr int PSM_ROWS = 64;
+// Row chunks of a long block of rows: after each of them a full union ends the work (see launch_predict).
+constexpr int64_t PRED_CHUNK0 = 256;
 
 template <typename T>
 static int launch_scores_mma(const float* t_scratch, const void* Bm, uint32_t* bits, int64_t B, int64_t r, int64_t I, float tau,
-                             size_t smem, cudaStream_t s) {
+                             int merge, cudaStream_t s) {
   const int64_t W = (I + 31) / 32;
-  STX_CUDA(launch_pdl(k_pred_scores_mma<T>, dim3(static_cast<unsigned>((W + PSM_WARPS - 1) / PSM_WARPS)), dim3(PSM_WARPS * 32), smem, s,
-                      t_scratch, static_cast<const T*>(Bm), bits, static_cast<int>(B), static_cast<int>(r), static_cast<int>(I), tau));
+  const int64_t tile = std::min<int64_t>(B, PSM_ROWS);
+  const size_t smem = static_cast<size_t>((tile + 7) / 8 * 8) * (r + 8) * sizeof(T);
+  STX_CUDA(launch_pdl(k_pred_scores_mma<T>, dim3(static_cast<unsigned>((W + PSM_WARPS - 1) / PSM_WARPS), static_cast<unsigned>((B + tile - 1) / tile)),
+                      dim3(PSM_WARPS * 32), smem, s, t_scratch, static_cast<const T*>(Bm), bits, static_cast<int>(B),
+                      static_cast<int>(tile), static_cast<int>(r), static_cast<int>(I), tau, merge));
   return STX_OK;
 }
 template <>
-int launch_scores_mma<float>(const float*, const void*, uint32_t*, int64_t, int64_t, int64_t, float, size_t, cudaStream_t) {
+int launch_scores_mma<float>(const float*, const void*, uint32_t*, int64_t, int64_t, int64_t, float, int, cudaStream_t) {
   return STX_ERR_UNSUPPORTED;
+}
+
+// t of B rows; rows of 8192 elements (16-bit; 4096 in fp32) and wider need more than 512 threads and a smaller tile.
+template <typename T>
+static int launch_t(const void* x, int64_t B, int64_t H, const void* A, int64_t r, float* t, uint32_t* zero_words, int64_t I,
+                    const uint32_t* skip_words, cudaStream_t s) {
+  const int threads = pred_t_threads(static_cast<int>(H), DT<T>::V);
+  const int W = static_cast<int>((I + 31) / 32);
+  const T* xt = static_cast<const T*>(x);
+  const T* At = static_cast<const T*>(A);
+  const int b = static_cast<int>(B), h = static_cast<int>(H), rr = static_cast<int>(r), ii = static_cast<int>(I);
+  // A block walks row tiles; about four blocks per SM in all, so that a chunk that finds the union full costs one
+  // wave of blocks and not one block per tile (4096 rows x 128 would be 16384 blocks, 60 us of empty ones).
+  auto rows_grid = [](int kt, int tiles) { return dim3(kt, std::min(tiles, std::max(1, (4 * num_sms() + kt - 1) / kt))); };
+  if (B < STX_GEMM_MIN_ROWS)
+    STX_CUDA(launch_pdl(k_pred_t<T>, dim3(rr, 1), dim3(threads), 0, s, xt, At, t, b, h, rr, zero_words, W));
+  else if (threads <= 512)
+    STX_CUDA(launch_pdl(k_pred_t_rows<T, 4, 8, 512>, rows_grid((rr + 3) / 4, (b + 7) / 8), dim3(threads), 0, s, xt, At, t, b, h, rr, zero_words, W,
+                        skip_words, ii));
+  else
+    STX_CUDA(launch_pdl(k_pred_t_rows<T, 2, 4, 1024>, rows_grid((rr + 1) / 2, (b + 3) / 4), dim3(threads), 0, s, xt, At, t, b, h, rr, zero_words, W,
+                        skip_words, ii));
+  return STX_OK;
 }
 
 template <typename T>
@@ -434,30 +573,44 @@ static int launch_predict(const void* x, int64_t B, int64_t H, const void* A, in
                           int64_t I, float tau, uint32_t* bits, void* scores_out, float* t_scratch,
                           int write_bits, unsigned parts, cudaStream_t s) {
   const unsigned groups = static_cast<unsigned>((B + PRED_BT - 1) / PRED_BT);
-  if (parts & 1u)
-    STX_CUDA(launch_pdl(k_pred_t<T>, dim3(static_cast<unsigned>(r), groups), dim3(pred_t_threads(static_cast<int>(H), DT<T>::V)),
-                        0, s, static_cast<const T*>(x), static_cast<const T*>(A), t_scratch, static_cast<int>(B),
-                        static_cast<int>(H), static_cast<int>(r), (groups > 1 && write_bits && (parts & 2u)) ? bits : nullptr,
-                        static_cast<int>((I + 31) / 32)));
   const int64_t W = (I + 31) / 32;
-  const size_t smem = static_cast<size_t>(std::min<int64_t>(B, PRED_BT)) * r * sizeof(float);
   // row blocks of 16-bit weights under the threshold rule: scores on the tensor pipe (the mask stays bit-exact)
-  const size_t smem_mma = static_cast<size_t>((B + 7) / 8 * 8) * (r + 8) * sizeof(T);
-  if ((parts & 2u) && sizeof(T) == 2 && write_bits && !scores_out && B >= 9 && r % 32 == 0 && r <= 32 * PSM_MAX_SPANS &&
-      smem_mma <= 48 * 1024 && std::isfinite(tau) && (reinterpret_cast<uintptr_t>(Bm) & 15) == 0)
-    return launch_scores_mma<T>(t_scratch, Bm, bits, B, r, I, tau, smem_mma, s);
-  if ((parts & 2u) && !(parts & 1u) && groups > 1 && write_bits) STX_CUDA(cudaMemsetAsync(bits, 0, W * sizeof(uint32_t), s));
-  if (parts & 2u)
+  const bool mma = sizeof(T) == 2 && write_bits && !scores_out && B >= 9 && r % 32 == 0 && r <= 32 * PSM_MAX_SPANS &&
+                   std::isfinite(tau) && (reinterpret_cast<uintptr_t>(Bm) & 15) == 0;
+  const bool merge = mma && B > PSM_ROWS;
+  if (merge && (parts & 3u) == 3u) {
+    // A long block of rows (a prompt) goes in chunks of 256, 1024, 4096, ... rows: the mask is the union over all
+    // rows, so a chunk that finds every bit set has nothing to do (8192 rows at 10 % density fill it within the
+    // first chunk), and full words are skipped one by one.
+    int64_t b0 = 0, n = PRED_CHUNK0;
+    while (b0 < B) {
+      const int64_t nb = std::min(n, B - b0);
+      float* t = t_scratch + b0 * r;
+      int rc = launch_t<T>(static_cast<const T*>(x) + b0 * H, nb, H, A, r, t, b0 == 0 ? bits : nullptr, I, b0 == 0 ? nullptr : bits, s);
+      if (rc == STX_OK) rc = launch_scores_mma<T>(t, Bm, bits, nb, r, I, tau, 1, s);
+      if (rc != STX_OK) return rc;
+      b0 += nb;
+      n *= 4;
+    }
+    return STX_OK;
+  }
+  if (parts & 1u) {
+    const int rc = launch_t<T>(x, B, H, A, r, t_scratch, ((merge || groups > 1 || !write_bits) && (parts & 2u)) ? bits : nullptr, I, nullptr, s);
+    if (rc != STX_OK) return rc;
+  }
+  if (!(parts & 2u)) return STX_OK;
+  if (!(parts & 1u) && (merge || (groups > 1 && !mma)) && write_bits) STX_CUDA(cudaMemsetAsync(bits, 0, W * sizeof(uint32_t), s));
+  if (mma) return launch_scores_mma<T>(t_scratch, Bm, bits, B, r, I, tau, merge ? 1 : 0, s);
+  const size_t smem = static_cast<size_t>(std::min<int64_t>(B, PRED_BT)) * r * sizeof(float);
   STX_CUDA(launch_pdl(k_pred_scores<T>, dim3(static_cast<unsigned>(W), groups), dim3(256), smem, s, t_scratch,
                       static_cast<const T*>(Bm), bits, static_cast<T*>(scores_out), static_cast<int>(B),
                       static_cast<int>(r), static_cast<int>(I), tau, write_bits));
-  
   return STX_OK;
 }
 
 // Implemented in stx_select.cu: per-row rules that need the whole score row.
 int mask_from_scores(const void* scores, int64_t B, int64_t I, int dtype, int method, float param,
-                     uint32_t* bits_out, void* scratch, cudaStream_t s);
+                     uint32_t* bits_out, bool zeroed, cudaStream_t s);
 
 // parts: bit 0 = t = A x, bit 1 = scores, threshold/selection and mask
 int predict_mask(const void* x, int64_t B, int64_t H, const void* A, int64_t r, const void* Bm, int64_t I,
@@ -478,8 +631,8 @@ int predict_mask(const void* x, int64_t B, int64_t H, const void* A, int64_t r, 
       break;
   }
   if (rc != STX_OK || method == STX_MASK_THRESHOLD || !(parts & 2u)) return rc;
-  void* sel_scratch = static_cast<char*>(scratch) + align_up(static_cast<size_t>(B) * r * sizeof(float), 256);
-  return mask_from_scores(scores_out, B, I, dtype, method, param, bits, sel_scratch, s);
+  // a call that ran both halves had its words cleared by the first kernel
+  return mask_from_scores(scores_out, B, I, dtype, method, param, bits, (parts & 1u) != 0, s);
 }
 
 }  // namespace stx

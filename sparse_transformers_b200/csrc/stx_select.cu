@@ -45,28 +45,78 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* s_w /*[32]*/
   return r;
 }
 
-// k-th largest (k >= 1) of n keys produced by key_at(i), exact, by 4 radix passes of 8 bits.
-// All threads of the block must call it; returns the key.  s_hist: 256 ints; s_pick: 2 ints.
-template <typename KeyAt>
+// Keys of a score in the order of order_key: the 16-bit types need their own 16 bits only (widening to float keeps the
+// order of all values), which halves the radix passes and lets a whole row of keys stay in shared memory.
+template <typename T> struct SelKey {
+  typedef uint16_t type;
+  static constexpr int BITS = 16;
+  static __device__ __forceinline__ uint32_t of(T v) {
+    const uint32_t u = *reinterpret_cast<const uint16_t*>(&v);
+    return (u & 0x8000u) ? (~u & 0xffffu) : (u | 0x8000u);
+  }
+  static __device__ __forceinline__ float value(uint32_t k) {
+    const uint16_t u = static_cast<uint16_t>((k & 0x8000u) ? (k & 0x7fffu) : ~k);
+    return DT<T>::to_f(*reinterpret_cast<const T*>(&u));
+  }
+};
+template <> struct SelKey<float> {
+  typedef uint32_t type;
+  static constexpr int BITS = 32;
+  static __device__ __forceinline__ uint32_t of(float v) { return order_key(v); }
+  static __device__ __forceinline__ float value(uint32_t k) { return key_value(k); }
+};
+
+constexpr int SEL_HISTS = 8;  // histograms of a block: a warp adds to number warp & 7, scores crowd into a few bins
+
+// k-th largest (k >= 1) of n keys of BITS bits produced by key_at(i), exact, by radix passes of 8 bits.
+// All threads of the block must call it; returns the key.  s_hist: SEL_HISTS x 256 ints; s_pick: 2 ints.
+// A pass: histogram, then warp 0 finds the bin (a lane sums 8 bins, a shuffle scan from the top finds the lane,
+// that lane walks its 8 bins); one thread walking 256 bins took 3 us of a pass.
+template <int BITS, typename KeyAt>
 __device__ __forceinline__ uint32_t block_kth_largest(KeyAt key_at, int n, int k, int* s_hist, int* s_pick) {
   uint32_t prefix = 0u, mask = 0u;
   int kk = k;
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) s_hist[i] = 0;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int* hist = s_hist + (wid % SEL_HISTS) * 256;
+  for (int shift = BITS - 8; shift >= 0; shift -= 8) {
+    for (int i = threadIdx.x; i < SEL_HISTS * 256; i += blockDim.x) s_hist[i] = 0;
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       const uint32_t key = key_at(i);
-      if ((key & mask) == prefix) atomicAdd(&s_hist[(key >> shift) & 255u], 1);
+      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = 0, b = 255;
-      for (; b > 0; --b) {
-        if (acc + s_hist[b] >= kk) break;
-        acc += s_hist[b];
+    if (wid == 0) {
+      int bin[8], sum = 0;  // bins 255 - 8 * lane - j, j = 0..7: the lanes go down from the top
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        bin[j] = 0;
+#pragma unroll
+        for (int q = 0; q < SEL_HISTS; ++q) bin[j] += s_hist[q * 256 + 255 - 8 * lane - j];
+        sum += bin[j];
       }
-      s_pick[0] = b;
-      s_pick[1] = kk - acc;
+      int inc = sum;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += v;
+      }
+      const int before = inc - sum;
+      // the first lane whose running total reaches kk (the last lane if none does)
+      const uint32_t reach = __ballot_sync(0xffffffffu, inc >= kk);
+      const int owner = reach ? __ffs(reach) - 1 : 31;
+      if (lane == owner) {
+        int acc = before, j = 0;
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+          if (j == q && acc + bin[q] < kk) {
+            acc += bin[q];
+            ++j;
+          }
+        }
+        s_pick[0] = 255 - 8 * lane - j;
+        s_pick[1] = kk - acc;
+      }
     }
     __syncthreads();
     prefix |= static_cast<uint32_t>(s_pick[0]) << shift;
@@ -84,6 +134,8 @@ k_mask_statistical(const T* __restrict__ scores, int I, float z, uint32_t* __res
   __shared__ double s_out;
   const T* s = scores + static_cast<size_t>(blockIdx.x) * I;
   const int t = threadIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
   double a = 0.0;
   for (int i = t; i < I; i += SEL_THREADS) a += static_cast<double>(DT<T>::to_f(s[i]));
   const double mean_d = block_sum_fixed(a, s_w, &s_out) / static_cast<double>(I);
@@ -100,66 +152,72 @@ k_mask_statistical(const T* __restrict__ scores, int I, float z, uint32_t* __res
   const float prod = DT<T>::round_f(__fmul_rn(std_r, z_r));
   const float cutoff = DT<T>::round_f(__fadd_rn(mean_r, prod));
   if (t == 0 && cutoff_out) cutoff_out[blockIdx.x] = cutoff;
-  const int W = (I + 31) >> 5;
-  for (int w = t; w < W; w += SEL_THREADS) {
-    uint32_t word = 0u;
-    const int n = min(32, I - w * 32);
-    for (int b = 0; b < n; ++b)
-      if (DT<T>::to_f(s[w * 32 + b]) > cutoff) word |= 1u << b;
-    if (word) atomicOr(&bits[w], word);
+  const int W = (I + 31) >> 5, lane = t & 31;
+  for (int w = t >> 5; w < W; w += SEL_THREADS / 32) {
+    const int i = w * 32 + lane;
+    const uint32_t word = __ballot_sync(0xffffffffu, i < I && DT<T>::to_f(s[i]) > cutoff);
+    if (lane == 0 && word) atomicOr(&bits[w], word);
   }
 }
 
-template <typename T>
+// Dynamic shared memory (KEYS_IN_SMEM): the row's keys.  A block reads its row once; the radix passes and the final
+// compare run on the keys.
+template <typename T, bool KEYS_IN_SMEM>
 __global__ void __launch_bounds__(SEL_THREADS)
 k_mask_topk(const T* __restrict__ scores, int I, int k, uint32_t* __restrict__ bits) {
-  __shared__ int s_hist[256];
+  typedef typename SelKey<T>::type Key;
+  extern __shared__ uint32_t s_keys[];
+  __shared__ int s_hist[SEL_HISTS * 256];
   __shared__ int s_pick[2];
-  __shared__ int s_wsum[32];
+  __shared__ int s_wties[32];
   __shared__ int s_above;
-  const T* s = scores + static_cast<size_t>(blockIdx.x) * I;
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  const uint32_t kth_key = block_kth_largest([&](int i) { return order_key(DT<T>::to_f(s[i])); }, I, k, s_hist, s_pick);
-  const float kth = key_value(kth_key);
-  // contiguous index ranges per thread keep the ascending order for the tie rule
-  const int per = (I + SEL_THREADS - 1) / SEL_THREADS;
-  const int lo = t * per, hi = min(I, lo + per);
-  int above = 0, ties = 0;
-  for (int i = lo; i < hi; ++i) {
-    const float v = DT<T>::to_f(s[i]);
-    above += v > kth;
-    ties += v == kth;
+  const int W = (I + 31) >> 5;
+  Key* s_key = reinterpret_cast<Key*>(s_keys);
+  pdl_wait();
+  pdl_launch_dependents();
+  const T* s = scores + static_cast<size_t>(blockIdx.x) * I;
+  if (KEYS_IN_SMEM) {
+    for (int i = t; i < I; i += SEL_THREADS) s_key[i] = static_cast<Key>(SelKey<T>::of(s[i]));
+    __syncthreads();
   }
+  auto key_at = [&](int i) -> uint32_t { return KEYS_IN_SMEM ? static_cast<uint32_t>(s_key[i]) : SelKey<T>::of(s[i]); };
+  const float kth = SelKey<T>::value(block_kth_largest<SelKey<T>::BITS>(key_at, I, k, s_hist, s_pick));
   if (t == 0) s_above = 0;
   __syncthreads();
-  atomicAdd(&s_above, above);
-  int inc = ties;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, inc, off);
-    if (lane >= off) inc += v;
+  // A warp owns a range of mask words.  First its scores above the k-th and equal to it are counted: ties are taken
+  // in ascending index order, so a warp has to know how many lie in front of its range.
+  const int per = (W + SEL_THREADS / 32 - 1) / (SEL_THREADS / 32);
+  const int lo = min(W, wid * per), hi = min(W, lo + per);
+  auto word_of = [&](int w, uint32_t& above, uint32_t& ties) {
+    const int i = w * 32 + lane;
+    const float v = i < I ? SelKey<T>::value(key_at(i)) : 0.f;
+    above = __ballot_sync(0xffffffffu, i < I && v > kth);
+    ties = __ballot_sync(0xffffffffu, i < I && v == kth);
+  };
+  int n_above = 0, n_ties = 0;
+  for (int w = lo; w < hi; ++w) {
+    uint32_t ab, ti;
+    word_of(w, ab, ti);
+    n_above += __popc(ab);
+    n_ties += __popc(ti);
   }
-  if (lane == 31) s_wsum[wid] = inc;
-  __syncthreads();
-  if (t == 0) {
-    int run = 0;
-    for (int w = 0; w < 32; ++w) {
-      const int v = s_wsum[w];
-      s_wsum[w] = run;
-      run += v;
-    }
+  if (lane == 0) {
+    atomicAdd(&s_above, n_above);
+    s_wties[wid] = n_ties;
   }
   __syncthreads();
-  int tie_rank = s_wsum[wid] + inc - ties;  // ties before this thread's range
-  const int ties_wanted = k - s_above;
-  for (int i = lo; i < hi; ++i) {
-    const float v = DT<T>::to_f(s[i]);
-    bool on = v > kth;
-    if (v == kth) {
-      on = tie_rank < ties_wanted;
-      ++tie_rank;
+  int left = k - s_above;  // ties this warp may still take
+  for (int w = 0; w < wid; ++w) left -= s_wties[w];
+  for (int w = lo; w < hi; ++w) {
+    uint32_t word, ti;
+    word_of(w, word, ti);
+    if (left > 0 && ti) {
+      const bool take = ((ti >> lane) & 1u) && __popc(ti & ((1u << lane) - 1u)) < left;
+      word |= __ballot_sync(0xffffffffu, take);
     }
-    if (on) atomicOr(&bits[i >> 5], 1u << (i & 31));
+    left -= __popc(ti);
+    if (lane == 0 && word) atomicOr(&bits[w], word);
   }
 }
 
@@ -168,7 +226,7 @@ template <typename T>
 __global__ void __launch_bounds__(SEL_THREADS)
 k_approx_topk(const T* __restrict__ scores, int I, int k, T* __restrict__ thr_out) {
   extern __shared__ uint32_t s_sk[];
-  __shared__ int s_hist[256];
+  __shared__ int s_hist[SEL_HISTS * 256];
   __shared__ int s_pick[2];
   __shared__ int s_n;
   const T* s = scores + static_cast<size_t>(blockIdx.x) * I;
@@ -203,29 +261,45 @@ k_approx_topk(const T* __restrict__ scores, int I, int k, T* __restrict__ thr_ou
   if (sketch_k < 1) sketch_k = 1;
   if (sketch_k > n) sketch_k = n;
   // the excluded -inf buckets sort last, so the rank among all buckets is the same
-  const uint32_t key = block_kth_largest([&](int i) { return s_sk[i]; }, S * width, static_cast<int>(sketch_k), s_hist, s_pick);
+  const uint32_t key = block_kth_largest<32>([&](int i) { return s_sk[i]; }, S * width, static_cast<int>(sketch_k), s_hist, s_pick);
   if (t == 0) thr_out[blockIdx.x] = DT<T>::from_f(__fmul_rn(key_value(key), 0.9f));
 }
 
+template <typename T>
+static int launch_topk(const void* scores, int64_t B, int64_t I, int k, uint32_t* bits, cudaStream_t s) {
+  const size_t keys = static_cast<size_t>(I) * sizeof(typename SelKey<T>::type);
+  constexpr size_t LIMIT = 200 * 1024;
+  const dim3 grid(static_cast<unsigned>(B)), block(SEL_THREADS);
+  const T* sc = static_cast<const T*>(scores);
+  if (keys > LIMIT) {  // rows of more than 51200 fp32 (102400 16-bit) scores: the keys are made from the scores in every pass
+    STX_CUDA(launch_pdl(k_mask_topk<T, false>, grid, block, 0, s, sc, static_cast<int>(I), k, bits));
+    return STX_OK;
+  }
+  static bool attr_set[64] = {};
+  int dev = 0;
+  STX_CUDA(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    STX_CUDA(cudaFuncSetAttribute(k_mask_topk<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(LIMIT)));
+    attr_set[dev] = true;
+  }
+  STX_CUDA(launch_pdl(k_mask_topk<T, true>, grid, block, keys, s, sc, static_cast<int>(I), k, bits));
+  return STX_OK;
+}
+
+// zeroed: `bits` was cleared by an earlier kernel of the same call
 int mask_from_scores(const void* scores, int64_t B, int64_t I, int dtype, int method, float param,
-                     uint32_t* bits_out, void* scratch, cudaStream_t s) {
-  (void)scratch;
+                     uint32_t* bits_out, bool zeroed, cudaStream_t s) {
   const size_t W = static_cast<size_t>((I + 31) / 32);
-  STX_CUDA(cudaMemsetAsync(bits_out, 0, W * sizeof(uint32_t), s));
-  const unsigned grid = static_cast<unsigned>(B);
+  if (!zeroed) STX_CUDA(cudaMemsetAsync(bits_out, 0, W * sizeof(uint32_t), s));
+  const dim3 grid(static_cast<unsigned>(B)), block(SEL_THREADS);
+  const int ii = static_cast<int>(I);
+  float* no_cutoff = nullptr;
   if (method == STX_MASK_STATISTICAL) {
     switch (dtype) {
-      case STX_F32:
-        k_mask_statistical<float><<<grid, SEL_THREADS, 0, s>>>(static_cast<const float*>(scores), static_cast<int>(I), param, bits_out, nullptr);
-        break;
-      case STX_F16:
-        k_mask_statistical<__half><<<grid, SEL_THREADS, 0, s>>>(static_cast<const __half*>(scores), static_cast<int>(I), param, bits_out, nullptr);
-        break;
-      default:
-        k_mask_statistical<__nv_bfloat16><<<grid, SEL_THREADS, 0, s>>>(static_cast<const __nv_bfloat16*>(scores), static_cast<int>(I), param, bits_out, nullptr);
-        break;
+      case STX_F32: STX_CUDA(launch_pdl(k_mask_statistical<float>, grid, block, 0, s, static_cast<const float*>(scores), ii, param, bits_out, no_cutoff)); break;
+      case STX_F16: STX_CUDA(launch_pdl(k_mask_statistical<__half>, grid, block, 0, s, static_cast<const __half*>(scores), ii, param, bits_out, no_cutoff)); break;
+      default: STX_CUDA(launch_pdl(k_mask_statistical<__nv_bfloat16>, grid, block, 0, s, static_cast<const __nv_bfloat16*>(scores), ii, param, bits_out, no_cutoff)); break;
     }
-    STX_LAUNCH_CHECK("k_mask_statistical");
     return STX_OK;
   }
   if (method == STX_MASK_TOPK) {
@@ -235,18 +309,10 @@ int mask_from_scores(const void* scores, int64_t B, int64_t I, int dtype, int me
       return STX_ERR_INVALID_ARG;
     }
     switch (dtype) {
-      case STX_F32:
-        k_mask_topk<float><<<grid, SEL_THREADS, 0, s>>>(static_cast<const float*>(scores), static_cast<int>(I), k, bits_out);
-        break;
-      case STX_F16:
-        k_mask_topk<__half><<<grid, SEL_THREADS, 0, s>>>(static_cast<const __half*>(scores), static_cast<int>(I), k, bits_out);
-        break;
-      default:
-        k_mask_topk<__nv_bfloat16><<<grid, SEL_THREADS, 0, s>>>(static_cast<const __nv_bfloat16*>(scores), static_cast<int>(I), k, bits_out);
-        break;
+      case STX_F32: return launch_topk<float>(scores, B, I, k, bits_out, s);
+      case STX_F16: return launch_topk<__half>(scores, B, I, k, bits_out, s);
+      default: return launch_topk<__nv_bfloat16>(scores, B, I, k, bits_out, s);
     }
-    STX_LAUNCH_CHECK("k_mask_topk");
-    return STX_OK;
   }
   set_error("mask rule %d needs no score pass", method);
   return STX_ERR_INVALID_ARG;
