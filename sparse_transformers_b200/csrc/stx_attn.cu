@@ -1,12 +1,11 @@
 // Decode-time glue of the LlamaSkip host around the sparse MLP (C ABI: stx_attn_decode,
 // stx_add_rmsnorm): one query token against the KV cache, and residual add + RMSNorm.
 //
-//   k_attn_decode   grid = query heads.  A CTA rotates its q head and the k head of its group
-//                   (rotate-half RoPE in fp32, rounded to the model dtype), appends k and v to
-//                   the cache (the first head of each group writes), scores the keys 0..pos
-//                   a warp per key with eight keys in flight, soft-maxes in fp32 and sums the
-//                   values with 16-byte chunks of the head dimension across threads.  The position is read from device memory, so a
-//                   captured CUDA graph can be replayed token after token.
+//   k_attn_decode   grid = groups of query heads that share a cache head x splits of the keys.  A CTA
+//                   rotates its q heads and the k head (rotate-half RoPE in fp32, rounded to the model
+//                   dtype), one CTA per cache head appends k and v, and every CTA streams its share of
+//                   the keys and values once for all of its query heads.  The position is read from
+//                   device memory, so a captured CUDA graph can be replayed token after token.
 //   k_add_rmsnorm   one CTA: h <- h + a (rounded to the model dtype), then
 //                   x = round(h * rsqrt(mean(h^2) + eps)) * w, the order of operations of
 //                   LlamaSkipRMSNorm (src/models/llama/modelling_llama_skip.py:39-44).
@@ -17,37 +16,10 @@
 #include <cstdlib>
 #include <cstring>
 
-#include <cooperative_groups.h>
-
 namespace stx {
-
-namespace cg = cooperative_groups;
 
 constexpr int ATT_THREADS = 512;
 constexpr int NORM_THREADS = 1024;
-
-template <typename T> struct Pair;
-template <> struct Pair<float> {
-  static __device__ __forceinline__ void load(const float* p, float& a, float& b) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    a = v.x;
-    b = v.y;
-  }
-};
-template <> struct Pair<__half> {
-  static __device__ __forceinline__ void load(const __half* p, float& a, float& b) {
-    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(p));
-    a = v.x;
-    b = v.y;
-  }
-};
-template <> struct Pair<__nv_bfloat16> {
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float& a, float& b) {
-    const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
-    a = v.x;
-    b = v.y;
-  }
-};
 
 // Block-wide max / sum over the block's threads; `red` has 32 floats.  Every thread gets the result.
 template <bool IS_MAX>
@@ -66,264 +38,250 @@ __device__ __forceinline__ float block_reduce(float v, float* red) {
   return r;
 }
 
-// `BYTES` consecutive bytes (4, 8, 16 or 32; aligned to min(BYTES, 16)) as 32-bit words.
-template <int BYTES>
-__device__ __forceinline__ void load_words(const void* p, uint32_t (&w)[BYTES / 4]) {
-  if constexpr (BYTES == 4) {
-    w[0] = *reinterpret_cast<const uint32_t*>(p);
-  } else if constexpr (BYTES == 8) {
-    const uint2 v = *reinterpret_cast<const uint2*>(p);
-    w[0] = v.x;
-    w[1] = v.y;
-  } else {
+// Workspace of stx_attn_decode: one arrival counter per group of heads (zero between launches), then per head and
+// split the unnormalised value sum [HD], the split's score maximum and its sum of exponentials.
+constexpr size_t ATT_COUNTER_BYTES = 4096;  // up to 1024 heads
+constexpr int ATT_MAX_SPLITS = 32;
+constexpr int ATT_KEYS_PER_SPLIT = 48;      // a split of fewer keys costs more in the merge than it saves
+__host__ __device__ inline int att_part_floats(int hd) { return hd + 2; }
+
+// Sums of v[0..N) over groups of G neighbouring lanes (powers of two).  A stage halves the values a lane keeps, as long
+// as there are two: about N + log2(G / N) shuffles instead of N log2(G).  Lane l of a group ends with value
+// l / (G / N) when G >= N, else with the N / G values from (l * N / G) on, in v[0..).
+template <int N, int G>
+__device__ __forceinline__ void group_sum_many(float (&v)[N], int lane) {
+  int n = N;
 #pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) {
-      const uint4 v = reinterpret_cast<const uint4*>(p)[i];
-      w[4 * i] = v.x;
-      w[4 * i + 1] = v.y;
-      w[4 * i + 2] = v.z;
-      w[4 * i + 3] = v.w;
+  for (int off = G / 2; off > 0; off >>= 1) {
+    if (n > 1) {
+      const bool hi = (lane & off) != 0;
+#pragma unroll
+      for (int j = 0; j < N / 2; ++j) {
+        if (j < n / 2) {
+          const float give = hi ? v[j] : v[j + n / 2];
+          const float keep = hi ? v[j + n / 2] : v[j];
+          v[j] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+      }
+      n /= 2;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
     }
   }
 }
-// Word i of a row of T as floats: one element for fp32, two for the 16-bit types.
-template <typename T> struct Words;
-template <> struct Words<float> {
-  static constexpr int EPW = 1;
-  static __device__ __forceinline__ void run(uint32_t w, float* f) { f[0] = __uint_as_float(w); }
-};
-template <> struct Words<__half> {
-  static constexpr int EPW = 2;
-  static __device__ __forceinline__ void run(uint32_t w, float* f) {
-    const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&w));
-    f[0] = t.x;
-    f[1] = t.y;
-  }
-};
-template <> struct Words<__nv_bfloat16> {
-  static constexpr int EPW = 2;
-  static __device__ __forceinline__ void run(uint32_t w, float* f) {
-    f[0] = __uint_as_float(w << 16);
-    f[1] = __uint_as_float(w & 0xffff0000u);
-  }
+
+// Shapes of the key stream: a row of HD elements is LPK lanes x CPT 16-byte chunks; a thread has U rows of keys and U of
+// values in flight, so a CTA takes TK keys at a time.
+template <typename T, int HD, int REP> struct AttShape {
+  static constexpr int V = DT<T>::V;
+  static constexpr int CH = HD / V;                 // 16-byte chunks of a row
+  static constexpr int LPK = CH < 32 ? CH : 32;
+  static constexpr int CPT = CH / LPK;
+  static constexpr int NG = ATT_THREADS / LPK;      // rows side by side
+  static constexpr int U = (sizeof(T) == 2 && REP > 1 ? 4 : 8) / CPT;  // what 128 registers hold without spilling
+  static constexpr int TK = NG * U;
 };
 
-// Workspace of stx_attn_decode: one arrival counter per head (zero between launches), then per
-// head and split the unnormalised value sum [HD], the split's score maximum and its sum of
-// exponentials.
-constexpr size_t ATT_COUNTER_BYTES = 4096;  // up to 1024 heads
-__host__ __device__ inline int att_part_floats(int hd) { return hd + 2; }
-
-// Grid (heads, splits): split s of a head takes an equal share of the cached keys (the last split
-// also the token's own key), so that one query head is read by several SMs.  CL: the splits of a
-// head form a thread-block cluster and split 0 merges the partial soft-maxes out of the others'
-// shared memory; otherwise they meet in the workspace and the split that arrives last at the
-// head's counter merges (a store, a fence, an atomic and a load more on the critical path).
-// Shared memory (floats): q_s[HD] | kn_s[HD] | vn_s[HD] | red[32] | acc_s[NG][HD] | sc[keys of the split + 1]
-template <typename T, int HD, bool CL>
-__global__ void __launch_bounds__(ATT_THREADS) k_attn_decode(const T* __restrict__ qkv, const float* __restrict__ cos_t,
-                                                              const float* __restrict__ sin_t,
-                                                              const long long* __restrict__ pos_dev, T* k_cache, T* v_cache,
-                                                              T* __restrict__ out, int nh, int nkv, long long max_len,
-                                                              float scale, unsigned char* workspace) {
-  constexpr int V = DT<T>::V;              // elements per 16 bytes
+// What bounds it: the KV bytes at long contexts, a chain of dependent trips (position, rows, merge) at short ones.
+// A CTA reads every key and value of its split once for its REP query heads (they share the cache head) with 16-byte
+// loads, U keys and U values per thread requested before the first is used and the next tile's requested as soon as
+// a tile's registers are free; soft-max over tiles with a running maximum.
+// 24 query heads on 8 cache heads of 128, 4000 tokens, fp16: four layers of norm, attention, projection and norm 136 -> 104 us
+// (a warp per key and one batch of keys at a time before, every query head reading the cache for itself: 18.5 us a launch).
+// The splits meet in the workspace: the last one to arrive at the group's counter merges.  Splits beyond what the
+// position can use leave at once.
+// Shared memory (floats): q_s[REP][HD] | kn_s[HD] | vn_s[HD] | sc[REP][TK] | red[16][REP][HD] | m[REP] l[REP] corr[REP]
+template <typename T, int HD, int REP>
+__global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restrict__ qkv, const float* __restrict__ cos_t,
+                                                                 const float* __restrict__ sin_t,
+                                                                 const long long* __restrict__ pos_dev, T* k_cache, T* v_cache,
+                                                                 T* __restrict__ out, int nh, int nkv, long long max_len,
+                                                                 float scale, unsigned char* workspace) {
+  typedef AttShape<T, HD, REP> S;
+  constexpr int V = S::V, LPK = S::LPK, CPT = S::CPT, NG = S::NG, U = S::U, TK = S::TK;
   constexpr int NW = ATT_THREADS / 32;
-  constexpr int E = HD / 32;               // elements of a key row per lane
-  constexpr int KB = E * sizeof(T);        // the same in bytes
-  constexpr int TPR = HD / V;              // threads per value row (16 bytes each)
-  constexpr int NG = ATT_THREADS / TPR;    // key groups of the value sum
-  constexpr int U = 8;                     // keys a warp has in flight
   extern __shared__ float sm[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* q_s = sm;
-  float* kn_s = q_s + HD;
+  float* kn_s = q_s + REP * HD;
   float* vn_s = kn_s + HD;
-  float* red = vn_s + HD;
-  float* acc_s = red + 32;
-  float* sc = acc_s + NG * HD;
+  float* sc = vn_s + HD;
+  float* red = sc + REP * TK;
+  float* m_s = red + NW * REP * HD;
+  float* l_s = m_s + REP;
+  float* corr_s = l_s + REP;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
+  pdl_launch_dependents();
   const long long pos = *pos_dev;
   if (pos < 0 || pos >= max_len) return;  // nothing sensible to do; the output is left as it was
-  const int h = blockIdx.x;
-  const int sp = blockIdx.y, NSP = gridDim.y;
-  const int rep = nh / nkv;
-  const int g = h / rep;
+  const int h0 = blockIdx.x * REP, g = h0 / (nh / nkv);
+  const int np = static_cast<int>(pos);   // cached keys
+  const int NSP = min(static_cast<int>(gridDim.y), np / ATT_KEYS_PER_SPLIT + 1);
+  const int sp = blockIdx.y;
+  if (sp >= NSP) return;
   T* kc = k_cache + static_cast<size_t>(g) * max_len * HD;
   T* vc = v_cache + static_cast<size_t>(g) * max_len * HD;
-  const int chunk = (static_cast<int>(pos) + NSP - 1) / NSP;  // cached keys per split
-  const int lo = min(sp * chunk, static_cast<int>(pos)), hi = min(lo + chunk, static_cast<int>(pos));
-  const bool own = sp == NSP - 1;   // this split also scores the token's own key
-  const T* ks = kc + static_cast<size_t>(lo) * HD;  // key j of the split is cached key lo + j
+  const int chunk = (np + NSP - 1) / NSP;
+  const int lo = min(sp * chunk, np), n = min(lo + chunk, np) - lo;  // key j of the split is cached key lo + j
+  const bool own = sp == NSP - 1;                                    // this split also takes the token's own key
+  const T* ks = kc + static_cast<size_t>(lo) * HD;
   const T* vs = vc + static_cast<size_t>(lo) * HD;
-  const int n = hi - lo + 1;        // sc[n - 1] is the own key's slot (unused unless `own`)
-  // The first batch of keys is requested before the rotation: it depends on the position only.
-  uint32_t kw[U][KB / 4];
-  auto load_keys = [&](int j0) {
+  const int ch = tid % LPK, grp = tid / LPK;
+
+  uint4 kr[U][CPT], vr[U][CPT];
+  auto load_tile = [&](const T* src, int j0, uint4 (&r)[U][CPT]) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int j = j0 + NW * u;
-      if (j < n - 1) load_words<KB>(reinterpret_cast<const char*>(ks + static_cast<size_t>(j) * HD) + lane * KB, kw[u]);
+      const int j = j0 + grp + NG * u;
+#pragma unroll
+      for (int c = 0; c < CPT; ++c)
+        r[u][c] = j < n ? ld_cached16(src + static_cast<size_t>(j) * HD + (ch + LPK * c) * V) : make_uint4(0, 0, 0, 0);
     }
   };
-  load_keys(warp);
+  load_tile(ks, 0, kr);
+  load_tile(vs, 0, vr);
 
-  if (tid < HD) {
+  for (int i = tid; i < (REP + 1) * HD; i += ATT_THREADS) {
     constexpr int half = HD / 2;
-    const int dp = tid < half ? tid + half : tid - half;
-    const float sign = tid < half ? -1.f : 1.f;
-    const float c = cos_t[pos * HD + tid], s = sin_t[pos * HD + tid];
-    const T* qrow = qkv + static_cast<size_t>(h) * HD;
-    const T* krow = qkv + static_cast<size_t>(nh + g) * HD;
-    const T* vrow = qkv + static_cast<size_t>(nh + nkv + g) * HD;
+    const int r = i / HD, d = i - r * HD;
+    const int dp = d < half ? d + half : d - half;
+    const float sign = d < half ? -1.f : 1.f;
+    const float c = cos_t[pos * HD + d], s = sin_t[pos * HD + d];
+    const T* row = qkv + static_cast<size_t>(r < REP ? h0 + r : nh + g) * HD;
     // x * cos + rotate_half(x) * sin: two rounded products, one rounded sum, then the model dtype
-    const T qr = DT<T>::from_f(__fadd_rn(__fmul_rn(DT<T>::to_f(qrow[tid]), c), __fmul_rn(sign * DT<T>::to_f(qrow[dp]), s)));
-    const T kr = DT<T>::from_f(__fadd_rn(__fmul_rn(DT<T>::to_f(krow[tid]), c), __fmul_rn(sign * DT<T>::to_f(krow[dp]), s)));
-    const T vr = vrow[tid];
-    q_s[tid] = DT<T>::to_f(qr);
-    kn_s[tid] = DT<T>::to_f(kr);
-    vn_s[tid] = DT<T>::to_f(vr);
-    if (h == g * rep && sp == 0) {  // one writer per group; every head of the group uses its own copy in shared memory
-      kc[pos * HD + tid] = kr;
-      vc[pos * HD + tid] = vr;
+    const T y = DT<T>::from_f(__fadd_rn(__fmul_rn(DT<T>::to_f(row[d]), c), __fmul_rn(sign * DT<T>::to_f(row[dp]), s)));
+    q_s[i] = DT<T>::to_f(y);  // row REP is kn_s
+    if (r == REP) {
+      const T v = qkv[static_cast<size_t>(nh + nkv + g) * HD + d];
+      vn_s[d] = DT<T>::to_f(v);
+      if (sp == 0 && h0 == g * (nh / nkv)) {  // one writer per cache head; the others use their own copy
+        kc[pos * HD + d] = y;
+        vc[pos * HD + d] = v;
+      }
     }
   }
   __syncthreads();
 
-  // ---- scores: a warp per key, lane l holds elements [l*E, l*E + E); U keys in flight per warp
-  float qf[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) qf[e] = q_s[lane * E + e];
-  float lmax = -INFINITY;
-  // the first batch of values, requested before the soft-max needs anything
-  const int grp = tid / TPR, ch = tid - grp * TPR;
-  uint4 raw[4];
-  auto load_values = [&](int j0) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + NG * u;
-      if (j < n - 1) raw[u] = *reinterpret_cast<const uint4*>(vs + static_cast<size_t>(j) * HD + ch * V);
+  // the running soft-max starts with the token's own key in the last split, with nothing in the others
+  if (warp < REP) {
+    float dot = 0.f;
+    for (int d = lane; d < HD; d += 32) dot = fmaf(q_s[warp * HD + d], kn_s[d], dot);
+    dot = warp_sum_xor(dot) * scale;
+    if (lane == 0) {
+      m_s[warp] = own ? dot : -INFINITY;
+      l_s[warp] = own ? 1.f : 0.f;
     }
-  };
-  load_values(grp);
-  for (int j0 = warp; j0 < n - 1; j0 += NW * U) {
-    if (j0 != warp) load_keys(j0);
+  }
+  float qf[REP][CPT * V], acc[REP][CPT * V];
+#pragma unroll
+  for (int r = 0; r < REP; ++r)
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        qf[r][c * V + v] = q_s[r * HD + (ch + LPK * c) * V + v];
+        acc[r][c * V + v] = own && grp == 0 ? vn_s[(ch + LPK * c) * V + v] : 0.f;
+      }
+
+  for (int j0 = 0; j0 < n; j0 += TK) {
+    // ---- scores of the tile
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+      float dot[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        dot[u] = 0.f;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          float f[V];
+          Unpack<T>::run(kr[u][c], f);
+#pragma unroll
+          for (int v = 0; v < V; ++v) dot[u] = fmaf(qf[r][c * V + v], f[v], dot[u]);
+        }
+      }
+      group_sum_many<U, LPK>(dot, lane);
+      constexpr int LPV = LPK / U;  // lanes that hold the same key's sum (LPK >= U in every instance)
+      const int u = ch / LPV;
+      if (ch % LPV == 0) sc[r * TK + grp + NG * u] = j0 + grp + NG * u < n ? dot[0] * scale : -INFINITY;
+    }
+    if (j0 + TK < n) load_tile(ks, j0 + TK, kr);
+    __syncthreads();
+    if (warp < REP) {  // a warp per query head
+      float* s = sc + warp * TK;
+      const float m_old = m_s[warp];
+      float m = m_old;
+#pragma unroll
+      for (int i = 0; i < TK / 32; ++i) m = fmaxf(m, s[lane + 32 * i]);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < TK / 32; ++i) {
+        const float p = m == -INFINITY ? 0.f : __expf(s[lane + 32 * i] - m);
+        s[lane + 32 * i] = p;
+        sum += p;
+      }
+      sum = warp_sum_xor(sum);
+      if (lane == 0) {
+        const float corr = m == -INFINITY ? 1.f : __expf(m_old - m);
+        m_s[warp] = m;
+        l_s[warp] = fmaf(l_s[warp], corr, sum);
+        corr_s[warp] = corr;
+      }
+    }
+    __syncthreads();
+    // ---- values of the tile
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+      const float corr = corr_s[r];
+#pragma unroll
+      for (int k = 0; k < CPT * V; ++k) acc[r][k] *= corr;
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int j = j0 + NW * u;
-      if (j < n - 1) {  // uniform over the warp
-        float dot = 0.f;
+      float p[REP];
 #pragma unroll
-        for (int i = 0; i < KB / 4; ++i) {
-          float f[Words<T>::EPW];
-          Words<T>::run(kw[u][i], f);
+      for (int r = 0; r < REP; ++r) p[r] = sc[r * TK + grp + NG * u];
 #pragma unroll
-          for (int e = 0; e < Words<T>::EPW; ++e) dot = fmaf(qf[i * Words<T>::EPW + e], f[e], dot);
-        }
-        dot = warp_sum_xor(dot) * scale;
-        if (lane == 0) sc[j] = dot;
-        lmax = fmaxf(lmax, dot);
-      }
-    }
-  }
-  if (warp == 0 && own) {  // the key of this token
-    float dot = 0.f;
-#pragma unroll
-    for (int e = 0; e < E; ++e) dot = fmaf(qf[e], kn_s[lane * E + e], dot);
-    dot = warp_sum_xor(dot) * scale;
-    if (lane == 0) sc[n - 1] = dot;
-    lmax = fmaxf(lmax, dot);
-  }
-  const float m = block_reduce<true>(lmax, red);  // its barriers also publish sc
-  const int nsc = own ? n : n - 1;
-  float lsum = 0.f;
-  for (int j = tid; j < nsc; j += ATT_THREADS) {
-    const float p = __expf(sc[j] - m);
-    sc[j] = p;
-    lsum += p;
-  }
-  const float denom = block_reduce<false>(lsum, red);
-
-  // ---- values: thread (grp, ch) sums p_j * v_j[16-byte chunk ch] over the keys j = grp, grp + NG, ...
-  float acc[V];
-#pragma unroll
-  for (int v = 0; v < V; ++v) acc[v] = 0.f;
-  for (int j0 = grp; j0 < n - 1; j0 += 4 * NG) {
-    if (j0 != grp) load_values(j0);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + NG * u;
-      if (j < n - 1) {
+      for (int c = 0; c < CPT; ++c) {
         float f[V];
-        Unpack<T>::run(raw[u], f);
-        const float p = sc[j];
+        Unpack<T>::run(vr[u][c], f);
 #pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] = fmaf(p, f[v], acc[v]);
+        for (int r = 0; r < REP; ++r)
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[r][c * V + v] = fmaf(p[r], f[v], acc[r][c * V + v]);
       }
     }
+    if (j0 + TK < n) load_tile(vs, j0 + TK, vr);
   }
-  if (grp == 0 && own) {
-    const float p = sc[n - 1];
+
+  // ---- sum over the row groups: the groups of a warp by shuffle, the warps through shared memory in warp order
 #pragma unroll
-    for (int v = 0; v < V; ++v) acc[v] = fmaf(p, vn_s[ch * V + v], acc[v]);
-  }
+  for (int r = 0; r < REP; ++r)
 #pragma unroll
-  for (int v = 0; v < V; ++v) acc_s[grp * HD + ch * V + v] = acc[v];
+    for (int k = 0; k < CPT * V; ++k) {
+      float a = acc[r][k];
+#pragma unroll
+      for (int off = LPK; off < 32; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+      if (lane < LPK) red[(warp * REP + r) * HD + (ch + LPK * (k / V)) * V + k % V] = a;
+    }
   __syncthreads();
-  if constexpr (CL) {
-    // this split's unnormalised sum, maximum and sum of exponentials, where the cluster can read them
-    if (tid < HD) {
-      float s = 0.f;
-      for (int k = 0; k < NG; ++k) s += acc_s[k * HD + tid];
-      q_s[tid] = s;  // the query is not needed any more
-    }
-    if (tid == 0) {
-      red[0] = m;
-      red[1] = denom;
-    }
-    cg::cluster_group cluster = cg::this_cluster();
-    cluster.sync();
-    if (sp == 0 && tid < HD) {
-      float pm[8], pl[8], pa[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (k < NSP) {
-          const float* rq = cluster.map_shared_rank(q_s, k);
-          const float* rr = cluster.map_shared_rank(red, k);
-          pm[k] = rr[0];
-          pl[k] = rr[1];
-          pa[k] = rq[tid];
-        }
-      }
-      float M = -INFINITY;
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (k < NSP) M = fmaxf(M, pm[k]);
-      float num = 0.f, den = 0.f;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (k < NSP) {
-          const float wgt = __expf(pm[k] - M);  // 0 for a split without keys (its maximum is -inf)
-          num = fmaf(wgt, pa[k], num);
-          den = fmaf(wgt, pl[k], den);
-        }
-      }
-      out[static_cast<size_t>(h) * HD + tid] = DT<T>::from_f(num / den);
-    }
-    cluster.sync();  // nobody leaves while split 0 may still read its shared memory
-    return;
-  }
-  int* counter = reinterpret_cast<int*>(workspace) + h;
-  float* part = reinterpret_cast<float*>(workspace + ATT_COUNTER_BYTES) + static_cast<size_t>(h) * NSP * att_part_floats(HD);
-  float* mine = part + static_cast<size_t>(sp) * att_part_floats(HD);
-  if (tid < HD) {
+  int* counter = reinterpret_cast<int*>(workspace) + blockIdx.x;
+  float* part = reinterpret_cast<float*>(workspace + ATT_COUNTER_BYTES);
+  auto part_of = [&](int split, int r) { return part + (static_cast<size_t>(h0 + r) * ATT_MAX_SPLITS + split) * att_part_floats(HD); };
+  for (int i = tid; i < REP * HD; i += ATT_THREADS) {
+    const int r = i / HD, d = i - r * HD;
     float s = 0.f;
-    for (int k = 0; k < NG; ++k) s += acc_s[k * HD + tid];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) s += red[w * REP * HD + i];
     if (NSP == 1) {
-      out[static_cast<size_t>(h) * HD + tid] = DT<T>::from_f(s / denom);
+      out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(s / l_s[r]);
     } else {
-      __stcg(mine + tid, s);
-      if (tid == 0) {
-        __stcg(mine + HD, m);
-        __stcg(mine + HD + 1, denom);
+      float* mine = part_of(sp, r);
+      __stcg(mine + d, s);
+      if (d == 0) {
+        __stcg(mine + HD, m_s[r]);
+        __stcg(mine + HD + 1, l_s[r]);
       }
     }
   }
@@ -340,31 +298,26 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attn_decode(const T* __restrict
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  if (tid < HD) {
-    float pm[8], pl[8], pa[8];  // all loads in flight together (at most 8 splits)
+  float* wgt = sc;  // [REP][ATT_MAX_SPLITS] weights (TK >= 64: the scores are not needed any more)
+  if (warp < REP) {
+    const float* pk = part_of(lane, warp);
+    const float pm = lane < NSP ? __ldcg(pk + HD) : -INFINITY, pl = lane < NSP ? __ldcg(pk + HD + 1) : 0.f;
+    float M = pm;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (k < NSP) {
-        const float* pk = part + k * att_part_floats(HD);
-        pm[k] = __ldcg(pk + HD);
-        pl[k] = __ldcg(pk + HD + 1);
-        pa[k] = __ldcg(pk + tid);
-      }
-    }
-    float M = -INFINITY;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (k < NSP) M = fmaxf(M, pm[k]);
-    float num = 0.f, den = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (k < NSP) {
-        const float wgt = __expf(pm[k] - M);  // 0 for a split without keys (its maximum is -inf)
-        num = fmaf(wgt, pa[k], num);
-        den = fmaf(wgt, pl[k], den);
-      }
-    }
-    out[static_cast<size_t>(h) * HD + tid] = DT<T>::from_f(num / den);
+    for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+    const float w = lane < NSP && pm != -INFINITY ? __expf(pm - M) : 0.f;  // 0 for a split without keys
+    wgt[warp * ATT_MAX_SPLITS + lane] = w;
+    const float den = warp_sum_xor(w * pl);
+    if (lane == 0) l_s[warp] = den;
+  }
+  __syncthreads();
+  for (int i = tid; i < REP * HD; i += ATT_THREADS) {
+    const int r = i / HD, d = i - r * HD;
+    const float* pk = part_of(0, r) + d;
+    float num = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < NSP; ++k) num = fmaf(wgt[r * ATT_MAX_SPLITS + k], __ldcg(pk + static_cast<size_t>(k) * att_part_floats(HD)), num);
+    out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(num / l_s[r]);
   }
 }
 
@@ -425,6 +378,8 @@ template <typename T>
 __global__ void __launch_bounds__(NORM_THREADS) k_add_rmsnorm(const T* h, const T* __restrict__ a, const T* __restrict__ w,
                                                                float eps, T* h_out, T* __restrict__ x_out, int H) {
   __shared__ float red[32];
+  pdl_wait();
+  pdl_launch_dependents();
   add_rmsnorm_block<T, NORM_MAX_H / NORM_THREADS>(h, a, w, eps, a ? h_out : nullptr, H, red, [&](int i, T x) { x_out[i] = x; });
 }
 
@@ -486,7 +441,9 @@ __global__ void __launch_bounds__(GEMV_THREADS) k_norm_gemv(const T* __restrict_
     }
   };
   uint4 bufa[GEMV_BATCH], bufb[GEMV_BATCH];
-  if (nitems > 0) load_item(0, bufa);  // in flight while the norm is computed
+  if (nitems > 0) load_item(0, bufa);  // weights: in flight while the preceding kernel ends and the norm is computed
+  pdl_wait();
+  pdl_launch_dependents();
   if (w_norm) {
     const bool first = blockIdx.x == 0;
     add_rmsnorm_block<T, NORM_MAX_H / GEMV_THREADS>(h, a, w_norm, eps, first ? h_out : nullptr, H, red, [&](int i, T x) {
@@ -533,7 +490,18 @@ __global__ void __launch_bounds__(GEMV_THREADS) k_norm_gemv_tma(const T* __restr
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // the small loads of the prologue go first: behind the bulk copies they would come back last
+  // The rows of W do not depend on the preceding kernel: they are requested while it ends.
+  if (mine > 0) {
+    if (lane == 0) mbar_expect_tx(&bar[warp], static_cast<uint32_t>(mine * row_bytes));
+    __syncwarp();
+    for (int k = lane; k < mine; k += 32) {
+      const int lr = warp + k * NW;
+      bulk_load(rows + static_cast<size_t>(lr) * row_bytes, W + static_cast<size_t>(r0 + lr) * H, static_cast<uint32_t>(row_bytes),
+                &bar[warp]);
+    }
+  }
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int MAXPT = NORM_MAX_H / GEMV_THREADS;
   NormRegs<MAXPT> nr_regs;
   uint4 xr[MAXPT / 4 + 1];
@@ -543,15 +511,6 @@ __global__ void __launch_bounds__(GEMV_THREADS) k_norm_gemv_tma(const T* __restr
 #pragma unroll
     for (int k = 0; k < MAXPT / 4 + 1; ++k)
       if (tid + k * GEMV_THREADS < nchunk) xr[k] = reinterpret_cast<const uint4*>(h)[tid + k * GEMV_THREADS];
-  }
-  if (mine > 0) {
-    if (lane == 0) mbar_expect_tx(&bar[warp], static_cast<uint32_t>(mine * row_bytes));
-    __syncwarp();
-    for (int k = lane; k < mine; k += 32) {
-      const int lr = warp + k * NW;
-      bulk_load(rows + static_cast<size_t>(lr) * row_bytes, W + static_cast<size_t>(r0 + lr) * H, static_cast<uint32_t>(row_bytes),
-                &bar[warp]);
-    }
   }
   if (w_norm) {
     const bool first = blockIdx.x == 0;
@@ -598,6 +557,13 @@ __global__ void __launch_bounds__(GEMV_THREADS) k_norm_gemv_tma(const T* __restr
 }
 
 template <typename T>
+static int launch_add_rmsnorm(const void* h, const void* a, const void* w, float eps, void* h_out, void* x_out, int H, cudaStream_t s) {
+  STX_CUDA(launch_pdl(k_add_rmsnorm<T>, dim3(1), dim3(NORM_THREADS), 0, s, static_cast<const T*>(h), static_cast<const T*>(a),
+                      static_cast<const T*>(w), eps, static_cast<T*>(h_out), static_cast<T*>(x_out), H));
+  return STX_OK;
+}
+
+template <typename T>
 static int launch_norm_gemv(const void* h, const void* a, const void* w_norm, float eps, const void* W, void* y, void* h_out,
                             void* x_out, int H, int N, cudaStream_t s) {
   const int warps = GEMV_THREADS / 32;
@@ -618,23 +584,51 @@ static int launch_norm_gemv(const void* h, const void* a, const void* w_norm, fl
       attr_set[dev] = true;
     }
     const unsigned grid = static_cast<unsigned>((N + rows_per_cta - 1) / rows_per_cta);
-    k_norm_gemv_tma<T><<<grid, GEMV_THREADS, smem_tma, s>>>(static_cast<const T*>(h), static_cast<const T*>(a),
-                                                            static_cast<const T*>(w_norm), eps, static_cast<const T*>(W),
-                                                            static_cast<T*>(y), static_cast<T*>(h_out), static_cast<T*>(x_out), H,
-                                                            N, rows_per_cta);
+    STX_CUDA(launch_pdl(k_norm_gemv_tma<T>, dim3(grid), dim3(GEMV_THREADS), smem_tma, s, static_cast<const T*>(h), static_cast<const T*>(a),
+                        static_cast<const T*>(w_norm), eps, static_cast<const T*>(W), static_cast<T*>(y), static_cast<T*>(h_out),
+                        static_cast<T*>(x_out), H, N, rows_per_cta));
   } else {
     const int want = (N + warps - 1) / warps;
     const unsigned grid = static_cast<unsigned>(std::min(want, sms));  // one CTA per SM: the norm is made once per CTA
-    k_norm_gemv<T><<<grid, GEMV_THREADS, row_bytes, s>>>(static_cast<const T*>(h), static_cast<const T*>(a),
-                                                         static_cast<const T*>(w_norm), eps, static_cast<const T*>(W),
-                                                         static_cast<T*>(y), static_cast<T*>(h_out), static_cast<T*>(x_out), H, N);
+    STX_CUDA(launch_pdl(k_norm_gemv<T>, dim3(grid), dim3(GEMV_THREADS), row_bytes, s, static_cast<const T*>(h), static_cast<const T*>(a),
+                        static_cast<const T*>(w_norm), eps, static_cast<const T*>(W), static_cast<T*>(y), static_cast<T*>(h_out),
+                        static_cast<T*>(x_out), H, N));
   }
-  STX_LAUNCH_CHECK("k_norm_gemv");
   return STX_OK;
 }
 
-// Splits of the keys per head: enough CTAs to cover the SMs once, at most 8.
-static int att_splits(int n_heads) { return std::max(1, std::min(8, (num_sms() + n_heads - 1) / n_heads)); }
+template <typename T, int HD, int REP>
+static int launch_attn(const void* qkv, const float* cos_t, const float* sin_t, const long long* pos, void* k_cache, void* v_cache,
+                       void* out, int nh, int nkv, long long max_len, float scale, void* workspace, cudaStream_t s) {
+  typedef AttShape<T, HD, REP> S;
+  constexpr int smem = static_cast<int>(sizeof(float) * ((REP + 2) * HD + REP * S::TK + ATT_THREADS / 32 * REP * HD + 3 * REP));
+  if (smem > 48 * 1024) {
+    static bool attr_set[64] = {};
+    int dev = 0;
+    STX_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+      STX_CUDA(cudaFuncSetAttribute(k_attn_decode<T, HD, REP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      attr_set[dev] = true;
+    }
+  }
+  const int groups = nh / REP;
+  const int nsp = std::max(1, std::min(ATT_MAX_SPLITS, num_sms() / groups));  // one CTA per SM
+  STX_CUDA(launch_pdl(k_attn_decode<T, HD, REP>, dim3(groups, nsp), dim3(ATT_THREADS), smem, s, static_cast<const T*>(qkv), cos_t, sin_t,
+                      pos, static_cast<T*>(k_cache), static_cast<T*>(v_cache), static_cast<T*>(out), nh, nkv, max_len, scale,
+                      static_cast<unsigned char*>(workspace)));
+  return STX_OK;
+}
+
+// Query heads of a CTA: the largest divisor of the heads per cache head up to 4.
+template <typename T, int HD>
+static int launch_attn_rep(const void* qkv, const float* cos_t, const float* sin_t, const long long* pos, void* k_cache, void* v_cache,
+                           void* out, int nh, int nkv, long long max_len, float scale, void* ws, cudaStream_t s) {
+  const int rep = nh / nkv;
+  if (rep % 4 == 0) return launch_attn<T, HD, 4>(qkv, cos_t, sin_t, pos, k_cache, v_cache, out, nh, nkv, max_len, scale, ws, s);
+  if (rep % 3 == 0) return launch_attn<T, HD, 3>(qkv, cos_t, sin_t, pos, k_cache, v_cache, out, nh, nkv, max_len, scale, ws, s);
+  if (rep % 2 == 0) return launch_attn<T, HD, 2>(qkv, cos_t, sin_t, pos, k_cache, v_cache, out, nh, nkv, max_len, scale, ws, s);
+  return launch_attn<T, HD, 1>(qkv, cos_t, sin_t, pos, k_cache, v_cache, out, nh, nkv, max_len, scale, ws, s);
+}
 
 }  // namespace stx
 
@@ -645,7 +639,7 @@ extern "C" {
 int stx_attn_decode_workspace_bytes(int n_heads, int head_dim, int64_t* bytes_out) {
   STX_CHECK_ARG(bytes_out, "stx_attn_decode_workspace_bytes: null pointer");
   STX_CHECK_ARG(n_heads > 0 && n_heads <= 1024 && head_dim > 0, "stx_attn_decode_workspace_bytes: bad shape");
-  *bytes_out = static_cast<int64_t>(ATT_COUNTER_BYTES + sizeof(float) * static_cast<size_t>(n_heads) * 8 * att_part_floats(head_dim));
+  *bytes_out = static_cast<int64_t>(ATT_COUNTER_BYTES + sizeof(float) * static_cast<size_t>(n_heads) * ATT_MAX_SPLITS * att_part_floats(head_dim));
   return STX_OK;
 }
 
@@ -662,59 +656,19 @@ int stx_attn_decode(const void* qkv, const float* cos_table, const float* sin_ta
                 "stx_attn_decode: %d query heads do not divide into %d key/value heads", n_heads, n_kv_heads);
   STX_CHECK_ARG(max_len > 0 && max_len <= 8192, "stx_attn_decode: max_len %lld outside 1..8192", static_cast<long long>(max_len));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int V = 16 / static_cast<int>(dtype_size(dtype));
-  const int nsp = att_splits(n_heads);
-  const size_t smem = sizeof(float) * (3 * head_dim + 32 + static_cast<size_t>(ATT_THREADS) * V +
-                                       static_cast<size_t>((max_len + nsp - 1) / nsp + 1));
   const float scale = 1.0f / sqrtf(static_cast<float>(head_dim));
   const long long* pos = reinterpret_cast<const long long*>(pos_dev);
-  const long long ml = max_len;
-  static int use_cluster = -1;  // STX_ATTN_MERGE=workspace selects the merge through global memory (A/B measurements)
-  if (use_cluster < 0) {
-    const char* e = getenv("STX_ATTN_MERGE");
-    use_cluster = (e && !strcmp(e, "workspace")) ? 0 : 1;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(n_heads, nsp, 1);
-  cfg.blockDim = dim3(ATT_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = static_cast<unsigned>(nsp);
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (use_cluster && nsp > 1) ? 1 : 0;
-#define STX_ATT_LAUNCH_CL(T, HD, CL)                                                                                       \
-  do {                                                                                                                     \
-    if (smem > 48 * 1024)                                                                                                  \
-      STX_CUDA(cudaFuncSetAttribute(k_attn_decode<T, HD, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));    \
-    STX_CUDA(cudaLaunchKernelEx(&cfg, k_attn_decode<T, HD, CL>, static_cast<const T*>(qkv), cos_table, sin_table, pos,     \
-                                static_cast<T*>(k_cache), static_cast<T*>(v_cache), static_cast<T*>(out), n_heads,         \
-                                n_kv_heads, ml, scale, static_cast<unsigned char*>(workspace)));                           \
-  } while (0)
-#define STX_ATT_LAUNCH(T, HD)                                   \
-  do {                                                          \
-    if (cfg.numAttrs) STX_ATT_LAUNCH_CL(T, HD, true);           \
-    else STX_ATT_LAUNCH_CL(T, HD, false);                       \
-  } while (0)
-#define STX_ATT_HD(T)                       \
-  do {                                      \
-    if (head_dim == 64) STX_ATT_LAUNCH(T, 64);        \
-    else if (head_dim == 128) STX_ATT_LAUNCH(T, 128); \
-    else STX_ATT_LAUNCH(T, 256);            \
-  } while (0)
+#define STX_ATT_ARGS qkv, cos_table, sin_table, pos, k_cache, v_cache, out, n_heads, n_kv_heads, static_cast<long long>(max_len), scale, workspace, s
+#define STX_ATT_HD(T)                                                                  \
+  (head_dim == 64 ? launch_attn_rep<T, 64>(STX_ATT_ARGS)                               \
+                  : head_dim == 128 ? launch_attn_rep<T, 128>(STX_ATT_ARGS) : launch_attn_rep<T, 256>(STX_ATT_ARGS))
   switch (dtype) {
-    case STX_F32: STX_ATT_HD(float); break;
-    case STX_F16: STX_ATT_HD(__half); break;
-    default: STX_ATT_HD(__nv_bfloat16); break;
+    case STX_F32: return STX_ATT_HD(float);
+    case STX_F16: return STX_ATT_HD(__half);
+    default: return STX_ATT_HD(__nv_bfloat16);
   }
 #undef STX_ATT_HD
-#undef STX_ATT_LAUNCH
-#undef STX_ATT_LAUNCH_CL
-  STX_LAUNCH_CHECK("k_attn_decode");
-  return STX_OK;
+#undef STX_ATT_ARGS
 }
 
 int stx_add_rmsnorm(const void* h, const void* a, const void* w, float eps, void* h_out, void* x_out, int64_t H, int dtype,
@@ -726,24 +680,10 @@ int stx_add_rmsnorm(const void* h, const void* a, const void* w, float eps, void
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int Hi = static_cast<int>(H);
   switch (dtype) {
-    case STX_F32:
-      k_add_rmsnorm<float><<<1, NORM_THREADS, 0, s>>>(static_cast<const float*>(h), static_cast<const float*>(a),
-                                                      static_cast<const float*>(w), eps, static_cast<float*>(h_out),
-                                                      static_cast<float*>(x_out), Hi);
-      break;
-    case STX_F16:
-      k_add_rmsnorm<__half><<<1, NORM_THREADS, 0, s>>>(static_cast<const __half*>(h), static_cast<const __half*>(a),
-                                                       static_cast<const __half*>(w), eps, static_cast<__half*>(h_out),
-                                                       static_cast<__half*>(x_out), Hi);
-      break;
-    default:
-      k_add_rmsnorm<__nv_bfloat16><<<1, NORM_THREADS, 0, s>>>(
-          static_cast<const __nv_bfloat16*>(h), static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(w), eps,
-          static_cast<__nv_bfloat16*>(h_out), static_cast<__nv_bfloat16*>(x_out), Hi);
-      break;
+    case STX_F32: return launch_add_rmsnorm<float>(h, a, w, eps, h_out, x_out, Hi, s);
+    case STX_F16: return launch_add_rmsnorm<__half>(h, a, w, eps, h_out, x_out, Hi, s);
+    default: return launch_add_rmsnorm<__nv_bfloat16>(h, a, w, eps, h_out, x_out, Hi, s);
   }
-  STX_LAUNCH_CHECK("k_add_rmsnorm");
-  return STX_OK;
 }
 
 int stx_norm_gemv(const void* h, const void* a, const void* w_norm, float eps, const void* W, void* y, void* h_out,
