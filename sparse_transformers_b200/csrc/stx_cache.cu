@@ -23,6 +23,8 @@ k_cache_plan(const uint32_t* __restrict__ new_bits, uint32_t* __restrict__ cur_b
              int32_t* __restrict__ active, int32_t* __restrict__ pos_of, int32_t* __restrict__ lists,
              int32_t* __restrict__ jobs, int32_t* __restrict__ state, uint32_t* __restrict__ stale, int lazy, int I) {
   extern __shared__ int32_t sm[];
+  pdl_wait();
+  pdl_launch_dependents();
   plan_block(new_bits, cur_bits, active, pos_of, lists, jobs, state, stale, lazy, I, sm);
 }
 
@@ -31,6 +33,8 @@ __global__ void __launch_bounds__(128)
 k_cache_copy_rows(const int32_t* __restrict__ jobs, const int32_t* __restrict__ active,
                   const int32_t* __restrict__ state, const void* pool0, const void* pool1,
                   const void* pool2, void* pk0, void* pk1, void* pk2, int nmat, int vec_per_row, int I) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int njobs = state[ST_NJOBS];
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -111,7 +115,7 @@ __global__ void k_fill_i32(int32_t* p, int32_t v, size_t n) {
 
 static size_t plan_smem_bytes(int64_t I) { return plan_smem_words(I) * sizeof(int32_t); }
 
-int cache_plan(stx_cache* c, const uint32_t* bits, cudaStream_t s, bool lazy) {
+int cache_plan(stx_cache* c, const uint32_t* bits, cudaStream_t s, bool lazy, bool pdl) {
   static bool attr_set[64] = {};
   int dev = 0;
   STX_CUDA(cudaGetDevice(&dev));
@@ -123,9 +127,8 @@ int cache_plan(stx_cache* c, const uint32_t* bits, cudaStream_t s, bool lazy) {
   // two mask words per thread at most; small index spaces use fewer threads (cheaper barriers)
   const int W = static_cast<int>((c->I + 31) / 32);
   const int threads = W <= 256 ? 256 : (W <= 512 ? 512 : PLAN_THREADS);
-  k_cache_plan<<<1, threads, plan_smem_bytes(c->I), s>>>(bits, c->cur_bits, c->active, c->pos_of, c->lists, c->jobs,
-                                                        c->state, c->stale, lazy ? 1 : 0, static_cast<int>(c->I));
-  STX_LAUNCH_CHECK("k_cache_plan");
+  STX_CUDA(launch_pdl_if(pdl, k_cache_plan, dim3(1), dim3(threads), plan_smem_bytes(c->I), s, bits, c->cur_bits, c->active, c->pos_of,
+                         c->lists, c->jobs, c->state, c->stale, lazy ? 1 : 0, static_cast<int>(c->I)));
   if (lazy) c->lazy_used = true;
   return STX_OK;
 }
@@ -174,30 +177,29 @@ int cache_flush(stx_cache* c, cudaStream_t s) {
   return cache_copy_rows(c, s);
 }
 
-int cache_copy_rows(stx_cache* c, cudaStream_t s) {
+int cache_copy_rows(stx_cache* c, cudaStream_t s, bool pdl) {
   const int nmat = c->has_gate ? 3 : 2;
   const int vec = static_cast<int>(c->row_bytes / 16);
   // small blocks with few registers: they fit next to the MLP kernels' CTAs when the cache is
   // maintained on a side stream
-  const int grid = num_sms() * 4;
-  if (c->has_gate) {
-    k_cache_copy_rows<<<grid, 128, 0, s>>>(c->jobs, c->active, c->state, c->pool_gate, c->pool_up,
-                                          c->pool_down, c->pk_gate, c->pk_up, c->pk_down, nmat, vec,
-                                          static_cast<int>(c->I));
-  } else {
-    k_cache_copy_rows<<<grid, 128, 0, s>>>(c->jobs, c->active, c->state, c->pool_up, c->pool_down, nullptr,
-                                          c->pk_up, c->pk_down, nullptr, nmat, vec, static_cast<int>(c->I));
-  }
-  STX_LAUNCH_CHECK("k_cache_copy_rows");
+  const dim3 grid(num_sms() * 4), block(128);
+  const void* none = nullptr;
+  void* none_out = nullptr;
+  if (c->has_gate)
+    STX_CUDA(launch_pdl_if(pdl, k_cache_copy_rows, grid, block, 0, s, c->jobs, c->active, c->state, c->pool_gate, c->pool_up, c->pool_down,
+                           c->pk_gate, c->pk_up, c->pk_down, nmat, vec, static_cast<int>(c->I)));
+  else
+    STX_CUDA(launch_pdl_if(pdl, k_cache_copy_rows, grid, block, 0, s, c->jobs, c->active, c->state, c->pool_up, c->pool_down, none, c->pk_up,
+                           c->pk_down, none_out, nmat, vec, static_cast<int>(c->I)));
   return STX_OK;
 }
 
 int cache_update_bits(stx_cache* c, const uint32_t* bits, cudaStream_t s) {
   int rc = cache_flush(c, s);  // rows left stale by earlier lazy plans come first
   if (rc != STX_OK) return rc;
-  rc = cache_plan(c, bits, s, false);
+  rc = cache_plan(c, bits, s, false, true);
   if (rc != STX_OK) return rc;
-  return cache_copy_rows(c, s);
+  return cache_copy_rows(c, s, true);
 }
 
 // cat[n] = [gate[n] | up[n] | down[n]] (nmat rows of vec 16-byte vectors each)

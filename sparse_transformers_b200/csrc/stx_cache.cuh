@@ -60,8 +60,9 @@ namespace stx {
 int cache_update_bits(stx_cache* c, const uint32_t* bits, cudaStream_t s);
 // Plan only (index arrays, job list, state); the caller moves the rows.
 // lazy: remember the rewritten slots in `stale` instead of queueing them for cache_copy_rows
-int cache_plan(stx_cache* c, const uint32_t* bits, cudaStream_t s, bool lazy = false);
-int cache_copy_rows(stx_cache* c, cudaStream_t s);
+// pdl: the launch may overlap the end of the preceding kernel of the same stream (no dependency on other streams)
+int cache_plan(stx_cache* c, const uint32_t* bits, cudaStream_t s, bool lazy = false, bool pdl = false);
+int cache_copy_rows(stx_cache* c, cudaStream_t s, bool pdl = false);
 int cache_flush(stx_cache* c, cudaStream_t s);  // rows of all stale slots (no-op when none are pending)
 int cache_read_state(stx_cache* c, cudaStream_t s);  // syncs; fills host_state
 int cache_ensure_cat(stx_cache* c, cudaStream_t s);  // allocates and fills pool_cat once (asynchronous fill)

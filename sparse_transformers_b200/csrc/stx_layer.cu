@@ -29,7 +29,7 @@ bool layer_b1_supported(int64_t B, int64_t H, int64_t I, int64_t r, int has_gate
 int layer_b1_forward(const void* x, int64_t B, int64_t H, int64_t I, const void* gate, const void* up, const void* down,
                      const float* t, const void* Bm, int64_t r, float tau, uint32_t* bits, void* out, int act,
                      int has_gate, int dtype, float* partial, int* xchg, int* status, unsigned parts, const stx_peer* peer,
-                     cudaStream_t s);
+                     const UpkeepArgs* plan, cudaStream_t s);
 size_t layer_bn_xchg_bytes();
 int peer_allreduce(const stx_peer* p, void* data, int64_t n, int dtype, cudaStream_t s);
 int mlp_forward(const void* x, int64_t B, int64_t H, const void* gate, const void* up, const void* down,
@@ -77,17 +77,17 @@ struct stx_stack {
   std::vector<void*> b1_scratch;    // persistent single-row kernel: counters, t and partial vectors per group of layers
   bool persistent = false;
   // Device status of the step (bounded waits that expired, bounds checks that skipped an access): the last
-  // node of the graph ORs the layers' status words into status_dev and copies it to the pinned status_host,
+  // node of the graph ORs the layers' status words and stores the result in the pinned status_host,
   // which the NEXT stx_stack_step call reads without synchronising.
   stx::UpkeepArgs* upkeep_args = nullptr;  // device [L]: the layers' caches for upkeep that runs inside the flow kernel
   int** status_ptrs = nullptr;  // device [L]
-  int* status_dev = nullptr;
   int* status_host = nullptr;
 };
 
 using namespace stx;
 
-// ORs the layers' device status words into one (error bits only).
+// ORs the layers' device status words into one (error bits only).  `out` is pinned host memory: a store of four bytes
+// instead of a copy node of its own behind this one (7 us a step).
 __global__ void k_stack_status(int* const* __restrict__ ptrs, int n, int* __restrict__ out) {
   int v = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) v |= *ptrs[i] & (DEV_TIMEOUT | DEV_BAD_INDEX);
@@ -199,6 +199,31 @@ static bool single_row_fusable(const stx_layer* l, int64_t B) {
          layer_b1_supported(B, c->H, c->I, l->r, c->has_gate, c->dtype, c->pool_gate, c->pool_up, c->pool_down, l->Bm);
 }
 
+// What another kernel needs to run the cache's upkeep itself.
+static UpkeepArgs cache_upkeep_args(const stx_cache* c, bool lazy) {
+  UpkeepArgs u = {};
+  u.cur_bits = c->cur_bits, u.active = c->active, u.pos_of = c->pos_of, u.lists = c->lists, u.jobs = c->jobs;
+  u.state = c->state, u.stale = c->stale, u.lazy = lazy ? 1 : 0;
+  if (c->has_gate) {
+    u.pool[0] = c->pool_gate, u.pool[1] = c->pool_up, u.pool[2] = c->pool_down;
+    u.pk[0] = c->pk_gate, u.pk[1] = c->pk_up, u.pk[2] = c->pk_down;
+  } else {
+    u.pool[0] = c->pool_up, u.pool[1] = c->pool_down;
+    u.pk[0] = c->pk_up, u.pk[1] = c->pk_down;
+  }
+  return u;
+}
+
+// 2..8 rows of 16-bit gated weights under a rule that needs whole score rows (top-k, statistical): the same kernel,
+// k_mlp_bn, with the finished mask instead of its own scores.  Against the gate/up and down kernels of the general
+// path (which it replaces there): 3 rows of 4096 x 11008, 10 % per row, 107 -> 59 us a
+// step together with the selection kernel of stx_select.cu (30 -> 10 us).
+static bool given_mask_fusable(const stx_layer* l, int64_t B) {
+  const stx_cache* c = l->cache;
+  return l->partial && B >= 2 && B <= l->partial_rows && l->gather && l->method != STX_MASK_THRESHOLD &&
+         layer_b1_supported(B, c->H, c->I, 0, c->has_gate, c->dtype, c->pool_gate, c->pool_up, c->pool_down, c->pool_up);
+}
+
 // One step with the cache maintenance (plan + row copies) optionally on a second stream.
 // With `gather` the MLP reads the active rows straight from the full pools through the list
 // of set mask bits, so it needs neither the index plan nor the copied rows: the differential
@@ -212,6 +237,7 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
   // One row under the threshold rule: scores, mask, gather and MLP of a neuron stay in one CTA.
   float* partial = single_row_fusable(l, B) ? l->partial : nullptr;
   const bool fuse = partial && (stages & STX_STAGE_PREDICT_MASK) && (stages & STX_STAGE_MLP) && x_mlp && out;
+  const bool given = !fuse && given_mask_fusable(l, B);
   if (stages & STX_STAGE_PREDICT) {
     STX_CHECK_ARG(x_pred, "stx_layer_step: x_pred is null");
     const unsigned pparts = ((stages & STX_STAGE_PREDICT_T) ? 1u : 0u) | (((stages & STX_STAGE_PREDICT_MASK) && !fuse) ? 2u : 0u);
@@ -228,6 +254,12 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
   const bool gather = l->gather && !big;
   const bool forked = side != s && gather;
   cudaStream_t cs = forked ? side : s;  // stream of the cache maintenance
+  // a whole step on one stream: the upkeep kernels may start while their predecessor ends
+  const bool pdl = !forked && stages == STX_STAGE_ALL;
+  // ... and the index plan runs in a block of the kernel that adds the partial outputs
+  const bool plan_with_sum = pdl && (fuse || given) && !(l->peer && l->peer->world > 1);
+  const UpkeepArgs upkeep = cache_upkeep_args(c, l->lazy);
+  if (plan_with_sum && l->lazy) c->lazy_used = true;
   const bool fork_needed = forked && (stages & (STX_STAGE_PLAN | STX_STAGE_COPY));
   if (fork_needed && !fuse) {
     STX_CUDA(cudaEventRecord(fork_ev, s));
@@ -237,7 +269,7 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
     const float* t = static_cast<const float*>(l->pred_scratch);
     if (stages & STX_STAGE_MLP_GATEUP) {
       rc = layer_b1_forward(x_mlp, B, c->H, c->I, c->pool_gate, c->pool_up, c->pool_down, t, l->Bm, l->r, l->param, l->bits,
-                            out, l->act, c->has_gate, c->dtype, partial, l->xchg, c->state + ST_STATUS, 1u, l->peer, s);
+                            out, l->act, c->has_gate, c->dtype, partial, l->xchg, c->state + ST_STATUS, 1u, l->peer, nullptr, s);
       if (rc != STX_OK) return rc;
     }
     if (fork_needed) {  // the mask exists once that kernel is done
@@ -246,7 +278,8 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
     }
     if (stages & STX_STAGE_MLP_DOWN) {
       rc = layer_b1_forward(x_mlp, B, c->H, c->I, c->pool_gate, c->pool_up, c->pool_down, t, l->Bm, l->r, l->param, l->bits,
-                            out, l->act, c->has_gate, c->dtype, partial, l->xchg, c->state + ST_STATUS, 2u, l->peer, s);
+                            out, l->act, c->has_gate, c->dtype, partial, l->xchg, c->state + ST_STATUS, 2u, l->peer,
+                            plan_with_sum ? &upkeep : nullptr, s);
       if (rc != STX_OK) return rc;
     }
   }
@@ -258,11 +291,11 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
     const bool plan_here = big ? (stages & STX_STAGE_MLP) != 0 : (stages & STX_STAGE_PLAN) != 0;
     const bool copy_here = big ? (stages & STX_STAGE_MLP) != 0 : (stages & STX_STAGE_COPY) != 0;
     if (plan_here) {
-      rc = cache_plan(c, l->bits, s);
+      rc = cache_plan(c, l->bits, s, false, pdl);
       if (rc != STX_OK) return rc;
     }
     if (copy_here) {
-      rc = cache_copy_rows(c, s);
+      rc = cache_copy_rows(c, s, pdl);
       if (rc != STX_OK) return rc;
     }
   }
@@ -276,7 +309,15 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
       if (rc != STX_OK) return rc;
     }
   }
-  if ((stages & STX_STAGE_MLP) && !fuse && !big) {
+  if ((stages & STX_STAGE_MLP) && given) {
+    STX_CHECK_ARG(x_mlp && out, "stx_layer_step: x_mlp/out is null");
+    const unsigned parts = ((stages & STX_STAGE_MLP_GATEUP) ? 1u : 0u) | ((stages & STX_STAGE_MLP_DOWN) ? 2u : 0u);
+    rc = layer_b1_forward(x_mlp, B, c->H, c->I, c->pool_gate, c->pool_up, c->pool_down, nullptr, nullptr, 0, 0.f, l->bits, out,
+                          l->act, c->has_gate, c->dtype, l->partial, l->xchg, c->state + ST_STATUS, parts, l->peer,
+                          plan_with_sum ? &upkeep : nullptr, s);
+    if (rc != STX_OK) return rc;
+  }
+  if ((stages & STX_STAGE_MLP) && !fuse && !big && !given) {
     STX_CHECK_ARG(x_mlp && out, "stx_layer_step: x_mlp/out is null");
     const unsigned parts = ((stages & STX_STAGE_MLP_GATEUP) ? 1u : 0u) | ((stages & STX_STAGE_MLP_DOWN) ? 2u : 0u);
     if (gather)
@@ -292,8 +333,8 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
     }
   }
   if (gather) {
-    if (stages & STX_STAGE_PLAN) {
-      rc = cache_plan(c, l->bits, cs, l->lazy);
+    if ((stages & STX_STAGE_PLAN) && !plan_with_sum) {
+      rc = cache_plan(c, l->bits, cs, l->lazy, pdl);
       if (rc != STX_OK) return rc;
     }
     if ((stages & STX_STAGE_COPY) && !l->lazy) {
@@ -306,7 +347,7 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
         ccs = side2;
         if (used_side2) *used_side2 = true;
       }
-      rc = cache_copy_rows(c, ccs);
+      rc = cache_copy_rows(c, ccs, pdl);
       if (rc != STX_OK) return rc;
     }
   }
@@ -387,7 +428,6 @@ int stx_stack_destroy(stx_stack_t* s) {
   for (void* p : s->b1_scratch) cudaFree(p);
   cudaFree(s->upkeep_args);
   cudaFree(s->status_ptrs);
-  cudaFree(s->status_dev);
   if (s->status_host) cudaFreeHost(s->status_host);
   cudaFree(s->x_in);
   cudaFree(s->out);
@@ -430,9 +470,8 @@ static int64_t stack_group_size(int64_t L) {
 
 // Last nodes of a step's graph: the layers' error bits -> one word -> pinned host memory.
 static int capture_status(stx_stack* s, cudaStream_t cs) {
-  k_stack_status<<<1, 32, 0, cs>>>(s->status_ptrs, static_cast<int>(s->layers.size()), s->status_dev);
+  k_stack_status<<<1, 32, 0, cs>>>(s->status_ptrs, static_cast<int>(s->layers.size()), s->status_host);
   STX_LAUNCH_CHECK("k_stack_status");
-  STX_CUDA(cudaMemcpyAsync(s->status_host, s->status_dev, sizeof(int), cudaMemcpyDeviceToHost, cs));
   return STX_OK;
 }
 
@@ -546,8 +585,6 @@ int stx_stack_create_stages(stx_stack_t** out, stx_layer_t* const* layers, int64
   if (e == cudaSuccess) e = cudaMalloc(&s->out, xbytes * L);
   if (e == cudaSuccess) e = cudaMemset(s->x_in, 0, xbytes);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->status_ptrs), sizeof(int*) * L);
-  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->status_dev), sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(s->status_dev, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&s->status_host), sizeof(int));
   if (e == cudaSuccess) {
     *s->status_host = 0;
@@ -603,20 +640,7 @@ int stx_stack_create_stages(stx_stack_t** out, stx_layer_t* const* layers, int64
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->upkeep_args), sizeof(UpkeepArgs) * L);
     if (e == cudaSuccess) {
       std::vector<UpkeepArgs> hu(L);
-      for (int64_t i = 0; i < L; ++i) {
-        const stx_cache* c = s->layers[i]->cache;
-        UpkeepArgs& u = hu[i];
-        u = UpkeepArgs{};
-        u.cur_bits = c->cur_bits, u.active = c->active, u.pos_of = c->pos_of, u.lists = c->lists, u.jobs = c->jobs;
-        u.state = c->state, u.stale = c->stale, u.lazy = s->layers[i]->lazy ? 1 : 0;
-        if (c->has_gate) {
-          u.pool[0] = c->pool_gate, u.pool[1] = c->pool_up, u.pool[2] = c->pool_down;
-          u.pk[0] = c->pk_gate, u.pk[1] = c->pk_up, u.pk[2] = c->pk_down;
-        } else {
-          u.pool[0] = c->pool_up, u.pool[1] = c->pool_down;
-          u.pk[0] = c->pk_up, u.pk[1] = c->pk_down;
-        }
-      }
+      for (int64_t i = 0; i < L; ++i) hu[i] = cache_upkeep_args(s->layers[i]->cache, s->layers[i]->lazy);
       e = cudaMemcpy(s->upkeep_args, hu.data(), sizeof(UpkeepArgs) * L, cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();  // cleared counters and per-neuron pools are in place before the first launch

@@ -3,6 +3,7 @@
 // projections on the tensor pipe), then the sum of the per-CTA partial vectors (k_partial_reduce,
 // k_partial_reduce4), which also carries the all-reduce of sharded layers.
 #include "stx_mlp_stream.cuh"
+#include "stx_cache_plan.cuh"
 
 #include <cooperative_groups.h>
 
@@ -59,6 +60,37 @@ constexpr int B1_LIST_CAP = 192;
 // c = g + 8*c4 and elements 4*v4 .. 4*v4+3 of the chunk (V elements per chunk, ceil(r/V/8) groups c4).
 __host__ __device__ inline size_t pred_t_smem_bytes(int B, int r, int V) {
   return r > 0 ? static_cast<size_t>(B) * ((r / V + 7) / 8) * 8 * V * sizeof(float) : 0;
+}
+
+// The CTA's active neurons in ascending order, from its nby mask bytes in s_bytes (complete for all threads): the ids
+// to s_my, their number to every thread.
+__device__ __forceinline__ int cta_list_bytes(const uint8_t* s_bytes, int nby, int32_t* s_my, int* s_nlocal) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = gridDim.x;
+  if (warp == 0) {
+    int carry = 0;
+    for (int base = 0; base < nby; base += 32) {
+      const int kk = base + lane;
+      uint32_t byte = kk < nby ? s_bytes[kk] : 0u;
+      const int cnt = __popc(byte);
+      int inc = cnt;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += v;
+      }
+      int pos = carry + inc - cnt;
+      while (byte) {
+        const int n = 8 * (static_cast<int>(blockIdx.x) + G * kk) + __ffs(byte) - 1;
+        byte &= byte - 1;
+        if (pos < B1_LIST_CAP) s_my[pos] = n;
+        ++pos;
+      }
+      carry += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) *s_nlocal = min(carry, B1_LIST_CAP);
+  }
+  __syncthreads();
+  return *s_nlocal;
 }
 
 // Predictor back half for the calling CTA's neurons (mask bytes blockIdx.x, + gridDim.x, ...),
@@ -159,31 +191,19 @@ __device__ __forceinline__ int cta_scores_and_list(const T* __restrict__ Bm, con
     run_pass(pass, wv0, ok0);
     if ((pass + 1) * 8 < nby) run_pass(pass + 1, wv1, ok1);
   }
-  if (warp == 0) {  // the CTA's active neurons in ascending order
-    int carry = 0;
-    for (int base = 0; base < nby; base += 32) {
-      const int kk = base + lane;
-      uint32_t byte = kk < nby ? s_bytes[kk] : 0u;
-      const int cnt = __popc(byte);
-      int inc = cnt;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += v;
-      }
-      int pos = carry + inc - cnt;
-      while (byte) {
-        const int n = 8 * (static_cast<int>(blockIdx.x) + G * kk) + __ffs(byte) - 1;
-        byte &= byte - 1;
-        if (pos < B1_LIST_CAP) s_my[pos] = n;
-        ++pos;
-      }
-      carry += __shfl_sync(0xffffffffu, inc, 31);
-    }
-    if (lane == 0) *s_nlocal = min(carry, B1_LIST_CAP);
-  }
+  return cta_list_bytes(s_bytes, nby, s_my, s_nlocal);
+}
+
+// The same for a mask that is there already (a rule that needs whole score rows): the CTA reads its bytes of it.
+// Contains the kernel's griddepcontrol wait.
+__device__ __forceinline__ int cta_list_given(const uint32_t* bits, int I, int32_t* s_my, uint8_t* s_bytes, int* s_nlocal) {
+  const int tid = threadIdx.x, G = gridDim.x, NBY = (I + 7) >> 3;
+  const int nby = NBY > static_cast<int>(blockIdx.x) ? (NBY - 1 - static_cast<int>(blockIdx.x)) / G + 1 : 0;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (tid < nby) s_bytes[tid] = __ldcg(reinterpret_cast<const uint8_t*>(bits) + blockIdx.x + G * tid);
   __syncthreads();
-  return *s_nlocal;
+  return cta_list_bytes(s_bytes, nby, s_my, s_nlocal);
 }
 
 template <typename T>
@@ -393,7 +413,10 @@ __global__ void __launch_bounds__(512, 1) k_mlp_b1(const MlpB1Args q) {
 //                batch rows, k = the (up to) 8 neurons of the tile (m16n8k8).  Warp w owns columns
 //                w*H/16 .. and keeps its H/16 x 8 outputs in registers; the A fragments come
 //                transposed out of the down rows with ldmatrix.trans; a is rounded to the model
-//                dtype for the B fragment (as the reference's own activations are).
+//                dtype for the B fragment (as the reference's own activations are).  GIVEN: a goes in
+//                as the sum of two numbers of the model dtype, a = hi + lo, with m16n8k16: k 0..7
+//                multiply hi and k 8..15 lo with the same A registers (16 or 22 mantissa bits); an
+//                fp16 tile whose largest |a| is out of range is scaled by a power of two meanwhile.
 // A buffer is re-filled with the next tile's rows as soon as its phase is over, so two of the three
 // are in flight or ready while the third is being read.  Filling all 16 tile rows matters: the
 // kernel's instruction stream is dominated by the fragment loads of x (64 KB per tile pass) and the
@@ -416,10 +439,16 @@ constexpr uint32_t BN_POLL_LIMIT = 1u << 20;
 constexpr int BN_MAX = 8;
 constexpr int BN_TN_MAX = 8;
 constexpr int BN_MT_MAX = 16;  // m-tiles of 16 columns per warp: H <= 16 * 16 * 16
-constexpr int BN_HEADER = 1024;                // [0,64) 3 mbarriers | [256,512) a_s [8 neurons][8 rows of the batch]
+constexpr int BN_HEADER = 1024;                // [0,64) 3 mbarriers | [256,512) a: hi, then lo, [4 neuron pairs][8 rows of the batch]
 constexpr int BN_RED_BYTES = 16 * 16 * 8 * 4;  // [warp][tile row][batch] fp32
 
-template <typename T>
+// Power of two that brings activations of up to `amax` into the range of fp16 (1 where they fit, and for infinities and NaN).
+__device__ __forceinline__ float bn_scale(float amax) {
+  return amax > 32768.f && amax < INFINITY ? exp2f(static_cast<float>(14 - ilogbf(amax))) : 1.f;
+}
+
+// GIVEN: the mask is finished (q.bits) and a keeps the accuracy of fp32, as in the kernels this variant stands in for.
+template <typename T, bool GIVEN>
 __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
   constexpr int V = DT<T>::V;
   static_assert(sizeof(T) == 2, "16-bit weights only");
@@ -437,7 +466,8 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
   uint64_t* bar_x = reinterpret_cast<uint64_t*>(smem);
   uint64_t* bar_y = bar_x + 1;
   uint64_t* bar_z = bar_x + 2;
-  uint32_t* a_pk = reinterpret_cast<uint32_t*>(smem + 256);  // [neuron pair][batch row]: (a[2k][b], a[2k+1][b]) in the model dtype
+  uint32_t* a_pk = reinterpret_cast<uint32_t*>(smem + 256);  // [hi, lo][neuron pair][batch row]: (a[2k][b], a[2k+1][b]) in the model dtype
+  __shared__ float s_amax[2];
   const size_t t_bytes = pred_t_smem_bytes(B, q.r, V);
   float* t_s = reinterpret_cast<float*>(smem + BN_HEADER);
   float* red_s = reinterpret_cast<float*>(smem + BN_HEADER + t_bytes);
@@ -466,8 +496,10 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
   // the exchange's epoch was written by this layer's previous launch: read it ahead of everything
   // (the barriers inside the front-end make it visible to all threads)
   if (balance && tid == 0) s_epoch = *reinterpret_cast<volatile int*>(q.xchg);
-  int nlocal = cta_scores_and_list<T>(static_cast<const T*>(q.Bm), q.t, t_s, B, q.r, p.I, q.tau, q.bits, s_my, s_nib,
-                                      s_bytes, &s_nlocal);
+  int nlocal;
+  if constexpr (GIVEN) nlocal = cta_list_given(q.bits, p.I, s_my, s_bytes, &s_nlocal);
+  else nlocal = cta_scores_and_list<T>(static_cast<const T*>(q.Bm), q.t, t_s, B, q.r, p.I, q.tau, q.bits, s_my, s_nib, s_bytes,
+                                       &s_nlocal);
   int niter = (nlocal + TN - 1) / TN;
   int epoch = 0;
   const int n_own = nlocal;
@@ -680,14 +712,35 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
         }
         a = apply_act(p.act, g) * u;
       }
-      const float a_next = __shfl_down_sync(0xffffffffu, a, 8);  // neuron e + 1, same batch row
-      if ((e & 1) == 0) a_pk[(e >> 1) * 8 + b] = MmaK8<T>::pack(a, a_next);
+      if constexpr (GIVEN) {
+        if (DT<T>::id == STX_F16) {
+          float m = fabsf(a);
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+          if (lane == 0) s_amax[warp] = m;
+          asm volatile("bar.sync 1, 64;" ::: "memory");
+          a *= bn_scale(fmaxf(s_amax[0], s_amax[1]));
+        }
+        const float hi = DT<T>::round_f(a);
+        const float lo = isinf(hi) ? 0.f : a - hi;
+        const float hi_next = __shfl_down_sync(0xffffffffu, hi, 8);  // neuron e + 1, same batch row
+        const float lo_next = __shfl_down_sync(0xffffffffu, lo, 8);
+        if ((e & 1) == 0) {
+          a_pk[(e >> 1) * 8 + b] = MmaK8<T>::pack(hi, hi_next);
+          a_pk[32 + (e >> 1) * 8 + b] = MmaK8<T>::pack(lo, lo_next);
+        }
+      } else {
+        const float a_next = __shfl_down_sync(0xffffffffu, a, 8);  // neuron e + 1, same batch row
+        if ((e & 1) == 0) a_pk[(e >> 1) * 8 + b] = MmaK8<T>::pack(a, a_next);
+      }
     }
     __syncthreads();  // a_pk complete
     // ---- phase 2
     if (!mbar_wait_bounded(bar_z, parity)) timed_out = true;
     {
-      const uint32_t bfrag = a_pk[tq * 8 + gq];  // B[k = 2tq, 2tq+1][n = gq]
+      const uint32_t bfrag = a_pk[tq * 8 + gq];                     // B[k = 2tq, 2tq+1][n = gq]
+      const uint32_t blo = GIVEN ? a_pk[32 + tq * 8 + gq] : 0u;     // B[k = 2tq + 8, 2tq + 9][n = gq]
+      const float scale = GIVEN && DT<T>::id == STX_F16 ? bn_scale(fmaxf(s_amax[0], s_amax[1])) : 1.f;
       // ldmatrix row of this lane: neuron lane & 7 (a missing row of a short buffer reads row 0, its a is 0),
       // 8-column group lane >> 3 of the 32 columns of an m-tile pair
       const int zr = (lane & 7) < TN ? (lane & 7) : 0;
@@ -697,8 +750,22 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
         if (2 * mp < MT) {
           uint32_t af[4];
           ldmatrix_x4_trans(af, zrow + static_cast<size_t>(mp) * 64);
-          MmaK8<T>::run(dacc[2 * mp], af[0], af[1], bfrag);
-          MmaK8<T>::run(dacc[2 * mp + 1], af[2], af[3], bfrag);
+          if constexpr (!GIVEN) {
+            MmaK8<T>::run(dacc[2 * mp], af[0], af[1], bfrag);
+            MmaK8<T>::run(dacc[2 * mp + 1], af[2], af[3], bfrag);
+          } else if (DT<T>::id == STX_F16 && scale != 1.f) {
+            float t0[4] = {0.f, 0.f, 0.f, 0.f}, t1[4] = {0.f, 0.f, 0.f, 0.f};
+            MmaOp<T>::run16(t0, af[0], af[1], af[0], af[1], bfrag, blo);
+            MmaOp<T>::run16(t1, af[2], af[3], af[2], af[3], bfrag, blo);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              dacc[2 * mp][k] += t0[k] / scale;
+              dacc[2 * mp + 1][k] += t1[k] / scale;
+            }
+          } else {
+            MmaOp<T>::run16(dacc[2 * mp], af[0], af[1], af[0], af[1], bfrag, blo);
+            MmaOp<T>::run16(dacc[2 * mp + 1], af[2], af[3], af[2], af[3], bfrag, blo);
+          }
         }
       }
     }
@@ -732,9 +799,28 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
 // (pa.world > 1: the layer is one shard of several GPUs) the column sums are then exchanged
 // over peer memory and added in rank order before the output is written: the all-reduce of the
 // sharded down projection costs no extra launch.
-template <typename T>
+// PLAN: one more block, the last, runs the index plan of the layer's cache (one row of 2048 x 8192 in fp32: 42 -> 37 us a step): the plan needs the mask only, which is as old as
+// the partial vectors, and takes about as long as the sum.
+struct PlanCall {
+  const uint32_t* bits;
+  UpkeepArgs u;
+  int I;
+};
+template <bool PLAN>
+__device__ __forceinline__ bool plan_in_last_block(const PlanCall& pc) {
+  if constexpr (PLAN) {
+    extern __shared__ int32_t plan_sm[];
+    if (blockIdx.x == gridDim.x - 1) {
+      plan_block(pc.bits, pc.u.cur_bits, pc.u.active, pc.u.pos_of, pc.u.lists, pc.u.jobs, pc.u.state, pc.u.stale, pc.u.lazy, pc.I, plan_sm);
+      return true;
+    }
+  }
+  return false;
+}
+
+template <typename T, bool PLAN>
 __global__ void __launch_bounds__(1024) k_partial_reduce(const float* __restrict__ partial, int G, int H, T* __restrict__ out,
-                                                         const __grid_constant__ PeerArgs pa) {
+                                                         const __grid_constant__ PeerArgs pa, const __grid_constant__ PlanCall pc) {
   __shared__ float s_r[32][33];
   const int hc = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + hc;
@@ -742,6 +828,7 @@ __global__ void __launch_bounds__(1024) k_partial_reduce(const float* __restrict
   const int c0 = grp * per, c1 = min(G, c0 + per);
   pdl_wait();
   pdl_launch_dependents();
+  if (plan_in_last_block<PLAN>(pc)) return;
   const bool shared = pa.world > 1;
   const int epoch = shared ? peer_epoch_begin(pa) : 0;
   float sum = 0.f;
@@ -768,9 +855,9 @@ __global__ void __launch_bounds__(1024) k_partial_reduce(const float* __restrict
 
 // Same sum for long vectors (several rows): a thread owns 4 consecutive columns (16-byte loads),
 // a block 128 columns x 32 groups of CTAs.  n must be a multiple of 128.
-template <typename T>
+template <typename T, bool PLAN>
 __global__ void __launch_bounds__(1024) k_partial_reduce4(const float* __restrict__ partial, int G, int n, T* __restrict__ out,
-                                                          const __grid_constant__ PeerArgs pa) {
+                                                          const __grid_constant__ PeerArgs pa, const __grid_constant__ PlanCall pc) {
   __shared__ float4 s_r[32][33];
   const int qc = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int h = (blockIdx.x * 32 + qc) * 4;
@@ -778,6 +865,7 @@ __global__ void __launch_bounds__(1024) k_partial_reduce4(const float* __restric
   const int c0 = grp * per, c1 = min(G, c0 + per);
   pdl_wait();
   pdl_launch_dependents();
+  if (plan_in_last_block<PLAN>(pc)) return;
   const bool shared = pa.world > 1;
   const int epoch = shared ? peer_epoch_begin(pa) : 0;
   float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -854,7 +942,42 @@ struct B1Pred {  // predictor back half fused into k_mlp_b1 (Bm == nullptr: not 
   uint32_t* bits = nullptr;
   int r = 0;
   float tau = 0.f;
+  int I = 0;
+  const UpkeepArgs* plan = nullptr;  // the index plan of the layer's cache, run next to the sum (host memory)
 };
+
+// Sum of the CTAs' partial vectors (four columns per thread with `wide`), with the cache's index plan in one more block
+// where the caller asks for it.
+template <typename T, bool PLAN>
+static int launch_reduce_plan(const float* partial, int G, int n, bool wide, void* out, const B1Pred& pr, const PlanCall& pc, cudaStream_t s) {
+  const size_t smem = PLAN ? plan_smem_words(pc.I) * sizeof(int32_t) : 0;
+  if (PLAN) {
+    static bool attr_set[64] = {};
+    int dev = 0;
+    STX_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+      const int most = static_cast<int>(plan_smem_words(MAX_I) * sizeof(int32_t));
+      STX_CUDA(cudaFuncSetAttribute(k_partial_reduce<T, PLAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      STX_CUDA(cudaFuncSetAttribute(k_partial_reduce4<T, PLAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      attr_set[dev] = true;
+    }
+  }
+  const unsigned grid = static_cast<unsigned>(wide ? n / 128 : (n + 31) / 32) + (PLAN ? 1 : 0);
+  if (wide)
+    STX_CUDA(launch_pdl(k_partial_reduce4<T, PLAN>, dim3(grid), dim3(1024), smem, s, partial, G, n, static_cast<T*>(out), pr.peer, pc));
+  else
+    STX_CUDA(launch_pdl(k_partial_reduce<T, PLAN>, dim3(grid), dim3(1024), smem, s, partial, G, n, static_cast<T*>(out), pr.peer, pc));
+  return STX_OK;
+}
+template <typename T>
+static int launch_reduce(const float* partial, int G, int n, bool wide, void* out, const B1Pred& pr, cudaStream_t s) {
+  if (!pr.plan) return launch_reduce_plan<T, false>(partial, G, n, wide, out, pr, PlanCall{}, s);
+  PlanCall pc = {};
+  pc.bits = pr.bits;
+  pc.u = *pr.plan;
+  pc.I = pr.I;
+  return launch_reduce_plan<T, true>(partial, G, n, wide, out, pr, pc, s);
+}
 
 template <typename T>
 static int launch_b1(const GateUpArgs& g, const void* down, float* partial, void* out, int grid, unsigned parts,
@@ -883,9 +1006,7 @@ static int launch_b1(const GateUpArgs& g, const void* down, float* partial, void
     attr_set[dev] = true;
   }
   if (parts & 1u) STX_CUDA(launch_pdl(k_mlp_b1<T>, dim3(grid), dim3(512), smem, s, q));
-  if (parts & 2u)
-    STX_CUDA(launch_pdl(k_partial_reduce<T>, dim3((g.H + 31) / 32), dim3(1024), 0, s, static_cast<const float*>(partial),
-                        grid, g.H, static_cast<T*>(out), pr.peer));
+  if (parts & 2u) return launch_reduce<T>(partial, grid, g.H, false, out, pr, s);
   return STX_OK;
 }
 
@@ -896,7 +1017,8 @@ static size_t bn_smem_budget() {
   if (!budget) {
     cudaFuncAttributes fa;
     size_t stat = 4096;
-    if (cudaFuncGetAttributes(&fa, k_mlp_bn<T>) == cudaSuccess) stat = fa.sharedSizeBytes;
+    if (cudaFuncGetAttributes(&fa, k_mlp_bn<T, false>) == cudaSuccess) stat = fa.sharedSizeBytes;
+    if (cudaFuncGetAttributes(&fa, k_mlp_bn<T, true>) == cudaSuccess) stat = std::max(stat, fa.sharedSizeBytes);
     budget = 227 * 1024 - (stat + 127) / 128 * 128;
   }
   return budget;
@@ -936,19 +1058,16 @@ static int launch_bn(const GateUpArgs& g, const void* down, float* partial, void
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    STX_CUDA(cudaFuncSetAttribute(k_mlp_bn<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    STX_CUDA(cudaFuncSetAttribute(k_mlp_bn<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(bn_smem_budget<T>())));
+    STX_CUDA(cudaFuncSetAttribute(k_mlp_bn<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(bn_smem_budget<T>())));
     attr_set[dev] = true;
   }
-  if (parts & 1u) STX_CUDA(launch_pdl(k_mlp_bn<T>, dim3(grid), dim3(512), smem, s, q));
+  if (parts & 1u) STX_CUDA(launch_pdl(pr.Bm ? k_mlp_bn<T, false> : k_mlp_bn<T, true>, dim3(grid), dim3(512), smem, s, q));
   if (parts & 2u) {
     const int n = g.B * g.H;  // the partials of a CTA are one vector [B][H]
-    if (n % 128 == 0)
-      STX_CUDA(launch_pdl(k_partial_reduce4<T>, dim3(n / 128), dim3(1024), 0, s, static_cast<const float*>(partial), grid, n,
-                          static_cast<T*>(out), pr.peer));
-    else
-      STX_CUDA(launch_pdl(k_partial_reduce<T>, dim3((n + 31) / 32), dim3(1024), 0, s, static_cast<const float*>(partial), grid,
-                          n, static_cast<T*>(out), pr.peer));
+    return launch_reduce<T>(partial, grid, n, n % 128 == 0, out, pr, s);
   }
   return STX_OK;
 }
@@ -1017,11 +1136,11 @@ int partial_sum(const float* partial, int G, int64_t n, void* out, int dtype, cu
   const PeerArgs none = {};
   const int nn = static_cast<int>(n);
   switch (dtype) {
-    case STX_F32: STX_CUDA(launch_pdl(k_partial_reduce4<float>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn, static_cast<float*>(out), none)); break;
-    case STX_F16: STX_CUDA(launch_pdl(k_partial_reduce4<__half>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn, static_cast<__half*>(out), none)); break;
+    case STX_F32: STX_CUDA(launch_pdl(k_partial_reduce4<float, false>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn, static_cast<float*>(out), none, PlanCall{})); break;
+    case STX_F16: STX_CUDA(launch_pdl(k_partial_reduce4<__half, false>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn, static_cast<__half*>(out), none, PlanCall{})); break;
     default:
-      STX_CUDA(launch_pdl(k_partial_reduce4<__nv_bfloat16>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn,
-                          static_cast<__nv_bfloat16*>(out), none));
+      STX_CUDA(launch_pdl(k_partial_reduce4<__nv_bfloat16, false>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn,
+                          static_cast<__nv_bfloat16*>(out), none, PlanCall{}));
       break;
   }
   return STX_OK;
@@ -1032,7 +1151,8 @@ bool layer_b1_supported(int64_t B, int64_t H, int64_t I, int64_t r, int has_gate
   if (B < 1 || B > BN_MAX) return false;
   const size_t es = dtype_size(dtype);
   const int V = static_cast<int>(16 / es);
-  if ((H * es) % 16 != 0 || H / V < 32 || r % V != 0 || r / V > 32 || H > (1 << 20) || I > (1 << 24))
+  // r == 0: the mask is given (2..8 rows only)
+  if ((H * es) % 16 != 0 || H / V < 32 || r % V != 0 || r / V > 32 || H > (1 << 20) || I > (1 << 24) || (r == 0 && B == 1))
     return false;
   const uintptr_t al = reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) |
                        reinterpret_cast<uintptr_t>(down) | reinterpret_cast<uintptr_t>(Bm);
@@ -1048,7 +1168,7 @@ bool layer_b1_supported(int64_t B, int64_t H, int64_t I, int64_t r, int has_gate
 int layer_b1_forward(const void* x, int64_t B, int64_t H, int64_t I, const void* gate, const void* up, const void* down,
                      const float* t, const void* Bm, int64_t r, float tau, uint32_t* bits, void* out, int act,
                      int has_gate, int dtype, float* partial, int* xchg, int* status, unsigned parts, const stx_peer* peer,
-                     cudaStream_t s) {
+                     const UpkeepArgs* plan, cudaStream_t s) {
   GateUpArgs a;
   a.x = x;
   a.gate = gate;
@@ -1074,6 +1194,8 @@ int layer_b1_forward(const void* x, int64_t B, int64_t H, int64_t I, const void*
   pr.r = static_cast<int>(r);
   pr.tau = tau;
   pr.xchg = xchg;
+  pr.I = static_cast<int>(I);
+  pr.plan = plan;
   if (peer && peer->world > 1) {
     if (!peer_args(peer, &pr.peer)) {
       set_error("stx_layer_step: the layer's peer object is not connected");
