@@ -29,31 +29,23 @@ k_cache_plan(const uint32_t* __restrict__ new_bits, uint32_t* __restrict__ cur_b
 }
 
 // One warp per (job, matrix): packed[m][pos] = pool[m][active[pos]], 16-byte vectors.
-__global__ void __launch_bounds__(128)
-k_cache_copy_rows(const int32_t* __restrict__ jobs, const int32_t* __restrict__ active,
-                  const int32_t* __restrict__ state, const void* pool0, const void* pool1,
-                  const void* pool2, void* pk0, void* pk1, void* pk2, int nmat, int vec_per_row, int I) {
+__global__ void __launch_bounds__(128) k_cache_copy_rows(const __grid_constant__ UpkeepArgs u, int nmat, int vec_per_row, int I) {
   pdl_wait();
   pdl_launch_dependents();
-  const int njobs = state[ST_NJOBS];
+  const int units = u.state[ST_NJOBS] * nmat;
   const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int units = njobs * nmat;
-  for (int u = warp; u < units; u += nwarps) {
-    const int job = u / nmat, m = u - job * nmat;
-    const int pos = jobs[job];
+  for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < units; k += nwarps) {
+    const int job = k / nmat, m = k - job * nmat;
+    const int pos = u.jobs[job];
     if (pos < 0 || pos >= I) continue;
-    const int src = active[pos];
+    const int src = u.active[pos];
     if (src < 0 || src >= I) continue;
-    const uint4* sp = reinterpret_cast<const uint4*>(m == 0 ? pool0 : (m == 1 ? pool1 : pool2)) +
-                      static_cast<size_t>(src) * vec_per_row;
-    uint4* dp = reinterpret_cast<uint4*>(m == 0 ? pk0 : (m == 1 ? pk1 : pk2)) +
-                static_cast<size_t>(pos) * vec_per_row;
+    const uint4* sp = static_cast<const uint4*>(u.pool[m]) + static_cast<size_t>(src) * vec_per_row;
+    uint4* dp = static_cast<uint4*>(u.pk[m]) + static_cast<size_t>(pos) * vec_per_row;
     int c = lane;
     for (; c + 96 < vec_per_row; c += 128) {
-      uint4 v0 = ld_stream16(sp + c), v1 = ld_stream16(sp + c + 32), v2 = ld_stream16(sp + c + 64),
-            v3 = ld_stream16(sp + c + 96);
+      const uint4 v0 = ld_stream16(sp + c), v1 = ld_stream16(sp + c + 32), v2 = ld_stream16(sp + c + 64), v3 = ld_stream16(sp + c + 96);
       st16(dp + c, v0);
       st16(dp + c + 32, v1);
       st16(dp + c + 64, v2);
@@ -182,15 +174,8 @@ int cache_copy_rows(stx_cache* c, cudaStream_t s, bool pdl) {
   const int vec = static_cast<int>(c->row_bytes / 16);
   // small blocks with few registers: they fit next to the MLP kernels' CTAs when the cache is
   // maintained on a side stream
-  const dim3 grid(num_sms() * 4), block(128);
-  const void* none = nullptr;
-  void* none_out = nullptr;
-  if (c->has_gate)
-    STX_CUDA(launch_pdl_if(pdl, k_cache_copy_rows, grid, block, 0, s, c->jobs, c->active, c->state, c->pool_gate, c->pool_up, c->pool_down,
-                           c->pk_gate, c->pk_up, c->pk_down, nmat, vec, static_cast<int>(c->I)));
-  else
-    STX_CUDA(launch_pdl_if(pdl, k_cache_copy_rows, grid, block, 0, s, c->jobs, c->active, c->state, c->pool_up, c->pool_down, none, c->pk_up,
-                           c->pk_down, none_out, nmat, vec, static_cast<int>(c->I)));
+  STX_CUDA(launch_pdl_if(pdl, k_cache_copy_rows, dim3(num_sms() * 4), dim3(128), 0, s, cache_upkeep_args(c, false), nmat, vec,
+                         static_cast<int>(c->I)));
   return STX_OK;
 }
 

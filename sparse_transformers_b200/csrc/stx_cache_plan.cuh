@@ -352,4 +352,19 @@ struct UpkeepArgs {
   int lazy;             // plan only: the rewritten slots go to the stale bitmap
 };
 
+// What another kernel needs to run the cache's upkeep itself.
+inline UpkeepArgs cache_upkeep_args(const stx_cache* c, bool lazy) {
+  UpkeepArgs u = {};
+  u.cur_bits = c->cur_bits, u.active = c->active, u.pos_of = c->pos_of, u.lists = c->lists, u.jobs = c->jobs;
+  u.state = c->state, u.stale = c->stale, u.lazy = lazy ? 1 : 0;
+  if (c->has_gate) {
+    u.pool[0] = c->pool_gate, u.pool[1] = c->pool_up, u.pool[2] = c->pool_down;
+    u.pk[0] = c->pk_gate, u.pk[1] = c->pk_up, u.pk[2] = c->pk_down;
+  } else {
+    u.pool[0] = c->pool_up, u.pool[1] = c->pool_down;
+    u.pk[0] = c->pk_up, u.pk[1] = c->pk_down;
+  }
+  return u;
+}
+
 }  // namespace stx

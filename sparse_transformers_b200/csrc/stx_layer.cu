@@ -23,7 +23,7 @@ void* mlp_prefill_region(void* scratch, int64_t B, int64_t H, int64_t K);
 bool prefill_wanted(int64_t B, int64_t H, int64_t K, int dtype, int has_gate);
 int prefill_forward(const void* x, int64_t B, int64_t H, const void* concat, const void* down_packed, int64_t K,
                     void* out, void* combined, int act, int dtype, void* scratch, int* status, const int* k_dev,
-                    cudaStream_t s);
+                    bool pdl, cudaStream_t s);
 bool layer_b1_supported(int64_t B, int64_t H, int64_t I, int64_t r, int has_gate, int dtype, const void* gate,
                         const void* up, const void* down, const void* Bm);
 int layer_b1_forward(const void* x, int64_t B, int64_t H, int64_t I, const void* gate, const void* up, const void* down,
@@ -106,7 +106,7 @@ int stx_cache_mlp_forward(stx_cache_t* c, const void* x, int64_t B, void* out, i
   if (rc != STX_OK) return rc;
   if (c->pk_gate && prefill_wanted(B, c->H, c->I, c->dtype, c->has_gate))
     return prefill_forward(x, B, c->H, c->pk_gate, c->pk_down, c->I, out, nullptr, act, c->dtype,
-                           mlp_prefill_region(scratch, B, c->H, c->I), c->state + ST_STATUS, c->state + ST_K, s);
+                           mlp_prefill_region(scratch, B, c->H, c->I), c->state + ST_STATUS, c->state + ST_K, true, s);
   return mlp_forward(x, B, c->H, c->pk_gate, c->pk_up, c->pk_down, c->state + ST_K, 0, c->I, 0, out, nullptr, act, c->has_gate,
                      c->dtype, scratch, c->state + ST_STATUS, 3u, nullptr, nullptr, nullptr, true, s);
 }
@@ -199,29 +199,28 @@ static bool single_row_fusable(const stx_layer* l, int64_t B) {
          layer_b1_supported(B, c->H, c->I, l->r, c->has_gate, c->dtype, c->pool_gate, c->pool_up, c->pool_down, l->Bm);
 }
 
-// What another kernel needs to run the cache's upkeep itself.
-static UpkeepArgs cache_upkeep_args(const stx_cache* c, bool lazy) {
-  UpkeepArgs u = {};
-  u.cur_bits = c->cur_bits, u.active = c->active, u.pos_of = c->pos_of, u.lists = c->lists, u.jobs = c->jobs;
-  u.state = c->state, u.stale = c->stale, u.lazy = lazy ? 1 : 0;
-  if (c->has_gate) {
-    u.pool[0] = c->pool_gate, u.pool[1] = c->pool_up, u.pool[2] = c->pool_down;
-    u.pk[0] = c->pk_gate, u.pk[1] = c->pk_up, u.pk[2] = c->pk_down;
-  } else {
-    u.pool[0] = c->pool_up, u.pool[1] = c->pool_down;
-    u.pk[0] = c->pk_up, u.pk[1] = c->pk_down;
-  }
-  return u;
-}
-
-// 2..8 rows of 16-bit gated weights under a rule that needs whole score rows (top-k, statistical): the same kernel,
-// k_mlp_bn, with the finished mask instead of its own scores.  Against the gate/up and down kernels of the general
+// Up to 8 rows under a rule that needs whole score rows (top-k, statistical): the same kernels with the finished mask
+// instead of their own scores.  One row: k_mlp_b1 on the listed bits, as the general path would, but with the index
+// plan next to the sum.  2..8 rows (16-bit gated weights): k_mlp_bn.  Against the gate/up and down kernels of the general
 // path (which it replaces there): 3 rows of 4096 x 11008, 10 % per row, 107 -> 59 us a
 // step together with the selection kernel of stx_select.cu (30 -> 10 us).
 static bool given_mask_fusable(const stx_layer* l, int64_t B) {
   const stx_cache* c = l->cache;
-  return l->partial && B >= 2 && B <= l->partial_rows && l->gather && l->method != STX_MASK_THRESHOLD &&
+  return l->partial && B <= l->partial_rows && l->gather && l->method != STX_MASK_THRESHOLD &&
          layer_b1_supported(B, c->H, c->I, 0, c->has_gate, c->dtype, c->pool_gate, c->pool_up, c->pool_down, c->pool_up);
+}
+
+// Row blocks on the tensor cores over the packed cache, then the shards' sum.
+static bool row_block(const stx_layer* l, int64_t B) {
+  const stx_cache* c = l->cache;
+  return c->pk_gate && !single_row_fusable(l, B) && prefill_wanted(B, c->H, c->I, c->dtype, c->has_gate);
+}
+static int row_block_mlp(stx_layer* l, const void* x, int64_t B, void* out, bool pdl, cudaStream_t s) {
+  stx_cache* c = l->cache;
+  int rc = prefill_forward(x, B, c->H, c->pk_gate, c->pk_down, c->I, out, nullptr, l->act, c->dtype,
+                           mlp_prefill_region(l->mlp_scratch, B, c->H, c->I), c->state + ST_STATUS, c->state + ST_K, pdl, s);
+  if (rc == STX_OK && l->peer && l->peer->world > 1) rc = peer_allreduce(l->peer, out, B * c->H, c->dtype, s);
+  return rc;
 }
 
 // One step with the cache maintenance (plan + row copies) optionally on a second stream.
@@ -250,7 +249,7 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
   // Row blocks of 9 and more (16-bit, gated): the packed cache IS the operand of two tensor-core
   // GEMMs, so its maintenance comes first, on the same stream; the GEMMs are shaped for all I
   // slots and follow the device-side K (no host read-back, graph-capturable).
-  const bool big = !fuse && c->pk_gate && prefill_wanted(B, c->H, c->I, c->dtype, c->has_gate);
+  const bool big = !fuse && row_block(l, B);
   const bool gather = l->gather && !big;
   const bool forked = side != s && gather;
   cudaStream_t cs = forked ? side : s;  // stream of the cache maintenance
@@ -301,13 +300,8 @@ static int layer_step_streams(stx_layer* l, const void* x_pred, const void* x_ml
   }
   if ((stages & STX_STAGE_MLP) && big) {
     STX_CHECK_ARG(x_mlp && out, "stx_layer_step: x_mlp/out is null");
-    rc = prefill_forward(x_mlp, B, c->H, c->pk_gate, c->pk_down, c->I, out, nullptr, l->act, c->dtype,
-                         mlp_prefill_region(l->mlp_scratch, B, c->H, c->I), c->state + ST_STATUS, c->state + ST_K, s);
+    rc = row_block_mlp(l, x_mlp, B, out, true, s);
     if (rc != STX_OK) return rc;
-    if (l->peer && l->peer->world > 1) {
-      rc = peer_allreduce(l->peer, out, B * c->H, c->dtype, s);
-      if (rc != STX_OK) return rc;
-    }
   }
   if ((stages & STX_STAGE_MLP) && given) {
     STX_CHECK_ARG(x_mlp && out, "stx_layer_step: x_mlp/out is null");
@@ -472,6 +466,42 @@ static int64_t stack_group_size(int64_t L) {
 static int capture_status(stx_stack* s, cudaStream_t cs) {
   k_stack_status<<<1, 32, 0, cs>>>(s->status_ptrs, static_cast<int>(s->layers.size()), s->status_host);
   STX_LAUNCH_CHECK("k_stack_status");
+  return STX_OK;
+}
+
+// A stack of row blocks: the predictor and the cache upkeep of a layer need the stack's input only, not the layer
+// before, so they run on two branches of their own (predictors; upkeep), ahead of the GEMMs, which leave them shared
+// memory and registers on every SM.  Layers that share an object (or a cache) stay serial.
+static bool row_blocks_ahead(const stx_stack* s, unsigned stages) {
+  if (stages != STX_STAGE_ALL) return false;
+  for (size_t i = 0; i < s->layers.size(); ++i) {
+    if (!row_block(s->layers[i], s->B)) return false;
+    for (size_t k = 0; k < i; ++k)
+      if (s->layers[k] == s->layers[i] || s->layers[k]->cache == s->layers[i]->cache) return false;
+  }
+  return true;
+}
+static int capture_row_blocks(stx_stack* s, cudaStream_t cs, cudaStream_t side, cudaStream_t side2) {
+  const int64_t L = static_cast<int64_t>(s->layers.size());
+  const size_t xbytes = static_cast<size_t>(s->B) * s->H * s->es;
+  STX_CUDA(cudaEventRecord(s->events[L], cs));
+  STX_CUDA(cudaStreamWaitEvent(side, s->events[L], 0));
+  for (int64_t i = 0; i < L; ++i) {
+    stx_layer* l = s->layers[i];
+    stx_cache* c = l->cache;
+    int rc = predict_mask(s->x_in, s->B, c->H, l->A, l->r, l->Bm, c->I, c->dtype, l->method, l->param, l->bits, l->scores,
+                          l->pred_scratch, 3u, side);
+    if (rc != STX_OK) return rc;
+    STX_CUDA(cudaEventRecord(s->events[L + 1 + i], side));
+    STX_CUDA(cudaStreamWaitEvent(side2, s->events[L + 1 + i], 0));
+    rc = cache_plan(c, l->bits, side2);
+    if (rc == STX_OK) rc = cache_copy_rows(c, side2, true);
+    if (rc != STX_OK) return rc;
+    STX_CUDA(cudaEventRecord(s->events[i], side2));
+    STX_CUDA(cudaStreamWaitEvent(cs, s->events[i], 0));
+    rc = row_block_mlp(l, s->x_in, s->B, static_cast<char*>(s->out) + i * xbytes, false, cs);
+    if (rc != STX_OK) return rc;
+  }
   return STX_OK;
 }
 
@@ -654,15 +684,18 @@ int stx_stack_create_stages(stx_stack_t** out, stx_layer_t* const* layers, int64
     for (cudaStream_t st : sides) cudaStreamDestroy(st);
   } else {
   e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
-  if (e == cudaSuccess) {
+  if (e == cudaSuccess && row_blocks_ahead(s, stages)) {
+    rc = capture_row_blocks(s, cs, side, side2);
+    if (rc == STX_OK) rc = capture_status(s, cs);
+    const cudaError_t e2 = cudaStreamEndCapture(cs, &s->graph);
+    if (rc == STX_OK && e2 != cudaSuccess) e = e2;
+  } else if (e == cudaSuccess) {
     bool forked = false, used2 = false;
     for (int64_t i = 0; i < L && rc == STX_OK; ++i) {
       stx_layer* l = s->layers[i];
       rc = layer_step_streams(l, s->x_in, s->x_in, B, static_cast<char*>(s->out) + i * xbytes, cs, side, s->events[i], stages,
                               side2, s->events[L + 1 + i], &used2);
-      const bool big = l->cache->pk_gate && !single_row_fusable(l, B) &&
-                       prefill_wanted(B, l->cache->H, l->cache->I, l->cache->dtype, l->cache->has_gate);
-      forked = forked || (l->gather && !big && (stages & (STX_STAGE_PLAN | STX_STAGE_COPY)));
+      forked = forked || (l->gather && !row_block(l, B) && (stages & (STX_STAGE_PLAN | STX_STAGE_COPY)));
     }
     if (rc == STX_OK && forked) {  // join
       cudaError_t ej = cudaEventRecord(s->events[L], side);

@@ -262,7 +262,7 @@ size_t prefill_scratch_bytes(int64_t B, int64_t H, int64_t K);
 bool prefill_wanted(int64_t B, int64_t H, int64_t K, int dtype, int has_gate);
 int prefill_forward(const void* x, int64_t B, int64_t H, const void* concat, const void* down_packed, int64_t K,
                     void* out, void* combined, int act, int dtype, void* scratch, int* status, const int* k_dev,
-                    cudaStream_t s);
+                    bool pdl, cudaStream_t s);
 
 constexpr int64_t PARTIAL_ROWS = 256;  // per-CTA partial output vectors of the batch-1 kernel (>= SM count)
 
@@ -414,7 +414,7 @@ int sparse_mlp_forward_impl(const void* x, int64_t B, int64_t H, const void* con
   if (scratch_has_partial && prefill_wanted(B, H, K, dtype, has_gate)) {
     // row blocks: the gathered weights form a dense contraction -> tcgen05 GEMMs
     return prefill_forward(x, B, H, concat_w, down_packed, K, down_buf, combined_buf, act, dtype,
-                           static_cast<char*>(scratch) + decode_scratch_bytes(B, H, K), nullptr, nullptr,
+                           static_cast<char*>(scratch) + decode_scratch_bytes(B, H, K), nullptr, nullptr, true,
                            static_cast<cudaStream_t>(stream));
   }
   const char* cw = static_cast<const char*>(concat_w);

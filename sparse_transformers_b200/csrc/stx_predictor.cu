@@ -559,6 +559,9 @@ static int launch_t(const void* x, int64_t B, int64_t H, const void* A, int64_t 
   auto rows_grid = [](int kt, int tiles) { return dim3(kt, std::min(tiles, std::max(1, (4 * num_sms() + kt - 1) / kt))); };
   if (B < STX_GEMM_MIN_ROWS)
     STX_CUDA(launch_pdl(k_pred_t<T>, dim3(rr, 1), dim3(threads), 0, s, xt, At, t, b, h, rr, zero_words, W));
+  else if (threads <= 512 && B <= 128)  // two blocks per SM, or one beside a GEMM CTA of a stack's layer before
+    STX_CUDA(launch_pdl(k_pred_t_rows<T, 2, 4, 1024>, rows_grid((rr + 1) / 2, (b + 3) / 4), dim3(threads), 0, s, xt, At, t, b, h, rr, zero_words, W,
+                        skip_words, ii));
   else if (threads <= 512)
     STX_CUDA(launch_pdl(k_pred_t_rows<T, 4, 8, 512>, rows_grid((rr + 3) / 4, (b + 7) / 8), dim3(threads), 0, s, xt, At, t, b, h, rr, zero_words, W,
                         skip_words, ii));

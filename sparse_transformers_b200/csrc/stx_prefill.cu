@@ -24,8 +24,8 @@
 //               (64 tokens, 8700 neurons of 4096: GEMM 1 57 -> 44 us).  Both CTAs' copies complete on the even CTA's barrier
 //   warp 1      even CTA: issues the MMAs from one lane; tcgen05.commit (multicast to both CTAs)
 //               releases a stage / publishes an accumulator.  Allocates and frees tensor memory.
-//   warps 2..5  epilogue: tcgen05.ld 32 lanes x 32 tokens; a warp's 32 lanes are neighbouring
-//               columns of the result, so every store is one contiguous 64- or 128-byte piece
+//   warps 2..5 and 8..11  epilogue, every other 32 tokens each: tcgen05.ld 32 lanes x 32 tokens; a
+//               warp's 32 lanes are neighbouring columns of the result, so every store is one contiguous 64- or 128-byte piece
 //               whatever the alignment of the row.
 // Edges are handled by TMA zero fill on loads and by masked stores; no load is multicast.
 // Every mbarrier wait is bounded; a role whose wait expired records DEV_TIMEOUT, stops, and the
@@ -41,14 +41,15 @@
 namespace stx {
 
 constexpr int PF_BK = 64;
-constexpr int PF_THREADS = 256;
+constexpr int PF_THREADS = 384;
 constexpr int PF_TW = 128;                               // neurons of a MODE 0 tile (64 per CTA)
 constexpr int PF_HW = 256;                               // columns of H of a MODE 1 tile (128 per CTA)
 constexpr int PF_MAX_N = 256;                            // tokens of a tile
 constexpr int PF_MAX_STAGES = 12;
 constexpr uint32_t PF_A_BYTES = 128 * PF_BK * 2;         // a CTA's A tile of one stage
-constexpr uint32_t PF_XCH_BYTES = 2 * 2 * 2 * 16 * 32 * 4;  // [warp pair][buffer][g|u][16 tokens][32 lanes] fp32
+constexpr uint32_t PF_XCH_BYTES = 2 * 2 * 2 * 16 * 32 * 4;  // [epilogue set][warp pair][g|u][16 tokens][32 lanes] fp32
 constexpr uint32_t PF_SMEM = 226 * 1024;
+constexpr uint32_t PF_SMEM_FEW = 148 * 1024;
 constexpr uint32_t PF_WAIT_LIMIT = 1u << 22;
 constexpr int PF_GROUP = 8;                              // token tiles that walk the weights together
 
@@ -70,6 +71,8 @@ struct PfArgs {
   // Optional device-side count of valid rows of the packed weights (a weight cache's K): MODE 0
   // covers *k_dev neurons rounded up to a k-block, zeros beyond *k_dev; MODE 1 stops its contraction there.
   const int* k_dev;
+  int early;           // MODE 1: the weights do not depend on the preceding kernel, fetch them while it ends
+  int tmem_cols;       // two accumulators of n_tok columns, as a power of two
   float* part;         // MODE 1 with splits: part[split][M][ld_out], summed by the caller in split order
 };
 
@@ -262,12 +265,12 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
     }
     for (int b = 0; b < 2; ++b) {
       pf_mbar_init(&acc_full[b], 1);
-      pf_mbar_init(&acc_empty[b], 8);  // four epilogue warps of either CTA
+      pf_mbar_init(&acc_empty[b], 16);  // eight epilogue warps of either CTA
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // tensor memory: this warp of both CTAs allocates, the same warps free
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pf_smem(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pf_smem(tmem_slot)), "r"(p.tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -275,15 +278,17 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();
-  pdl_launch_dependents();
+  if (!(MODE == 1 && p.early && (warp == 0 || warp == 6))) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
 
   const uint32_t full0 = pf_mapa(full, 0);  // the even CTA's barriers
   const int k_valid = p.k_dev ? min(*p.k_dev, MODE == 0 ? p.N : p.Kd) : (MODE == 0 ? p.N : p.Kd);
   const PfPlan plan = pf_plan<MODE>(p, k_valid);
   bool timed_out = false;
 
-  if (warp == 0 || warp >= 6) {
+  if (warp == 0 || warp == 6 || warp == 7) {
     // ------------------------------------------------------------------ TMA producers
     if (lane == 0) {
       const int part = warp == 0 ? 0 : warp - 5;  // 0, 1: the halves of the A tile, 2: tokens
@@ -299,8 +304,11 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
         const int tok = t.tok0 + static_cast<int>(rank) * (p.n_tok / 2);
         const CUtensorMap* map = part == 2 ? &tmB : &tmA.m[MODE == 0 && box > 1 ? box - 1 : 0];
         const bool issue = part == 2 || MODE == 1 || box > 0;
-        int k = t.kb_lo * PF_BK;
-        for (int kb = 0; kb < t.nkb; ++kb, k += PF_BK) {
+        // One token tile: all pairs stream weights at once, and rows of a power of two of bytes would have every one of
+        // them ask for the same columns at the same time; each starts at another k block instead (GEMM 1 of 64 tokens,
+        // 8700 neurons of 4096: 44.4 -> 41.5 us)
+        int k = (MODE == 0 && p.even ? (it * 37) % t.nkb : t.kb_lo) * PF_BK;
+        for (int kb = 0; kb < t.nkb; ++kb) {
           if (!pf_wait(&empty[s], phase)) {
             timed_out = true;
             break;
@@ -312,6 +320,8 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
             else if (MODE == 0) pf_tma_2d(dst, map, k, m0, full0 + s * 8);
             else pf_tma_2d(dst, map, m0, k, full0 + s * 8);
           }
+          k += PF_BK;
+          if (MODE == 0 && k >= t.nkb * PF_BK) k = 0;
           if (++s == S) {
             s = 0;
             phase ^= 1;
@@ -348,7 +358,7 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
           const uint64_t da = pf_smem_desc(st, MODE == 0 ? 16 : 8192), db = pf_smem_desc(st + PF_A_BYTES, 16);
 #pragma unroll
           for (int kk = 0; kk < PF_BK / 16; ++kk)
-            pf_mma(tmem_base + buf * PF_MAX_N, da + (kk * A_STEP >> 4), db + (kk * 32 >> 4), idesc, (kb | kk) != 0);
+            pf_mma(tmem_base + buf * p.n_tok, da + (kk * A_STEP >> 4), db + (kk * 32 >> 4), idesc, (kb | kk) != 0);
           pf_commit(&empty[s]);
           if (++s == S) {
             s = 0;
@@ -361,8 +371,10 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue warps 2..5
+    // ------------------------------------------------------------------ epilogue warps 2..5, 8..11
     const int lg = warp & 3;  // TMEM lane group this warp may read
+    const int set = warp >> 3;
+    const int pair_bar = 1 + (lg & 1) + 2 * set;  // the gate and the up warp of the same neurons
     T* out = static_cast<T*>(p.a_out);
     T* comb = static_cast<T*>(p.combined);
     const uint32_t acc_empty0[2] = {pf_mapa(&acc_empty[0], 0), pf_mapa(&acc_empty[1], 0)};
@@ -379,29 +391,28 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
               "{\n\t.reg .pred a, b;\n\tsetp.ne.s32 a, %1, 0;\n\t"
               "barrier.cta.red.or.pred b, %2, 64, a;\n\tselp.s32 %0, 1, 0, b;\n\t}"
               : "=r"(dead)
-              : "r"(dead), "r"(1 + (lg & 1))
+              : "r"(dead), "r"(pair_bar)
               : "memory");
           timed_out = dead != 0;
         }
         if (timed_out) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + buf * PF_MAX_N;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + buf * p.n_tok;
       if (MODE == 0) {
         const int nl = (lg & 1) * 32 + lane;  // neuron inside the CTA's share
         const int j = t.m0 + (rank ? t.m_rows0 : 0) + nl;
         const bool mine = nl < (rank ? t.m_rows1 : t.m_rows0) && j < plan.cover;
         const bool is_up = lg >= 2;
-        float* xp = xch + (lg & 1) * 2048;
+        float* xp = xch + (2 * set + (lg & 1)) * 1024;
+        float* give = xp + (is_up ? 512 : 0);
+        const float* take = xp + (is_up ? 0 : 512);
         // gate warps finish tokens 0..15 of a chunk, up warps tokens 16..31: each hands the other half over
 #pragma unroll 1
-        for (int c = 0; c < p.n_tok; c += 32) {
-          if (c >= ntok) break;
+        for (int c = 32 * set; c < ntok; c += 64) {
           float v[32];
           pf_ld32(taddr + c, v);
-          float* xb = xp + ((c >> 5) & 1) * 1024;
-          float* give = xb + (is_up ? 512 : 0);
-          const float* take = xb + (is_up ? 0 : 512);
+          if (c >= 64) asm volatile("barrier.cta.sync %0, 64;" ::"r"(pair_bar) : "memory");  // the last chunk has been read
           if (is_up) {
 #pragma unroll
             for (int e = 0; e < 16; ++e) give[e * 32 + lane] = v[e];
@@ -409,7 +420,7 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
 #pragma unroll
             for (int e = 0; e < 16; ++e) give[e * 32 + lane] = v[16 + e];
           }
-          asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + (lg & 1)) : "memory");
+          asm volatile("barrier.cta.sync %0, 64;" ::"r"(pair_bar) : "memory");
           if (mine) {
             const int tb = c + (is_up ? 16 : 0);
             const size_t row0 = static_cast<size_t>(t.tok0 + tb);
@@ -432,8 +443,7 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
       } else {
         const int col = t.m0 + static_cast<int>(rank) * 128 + lg * 32 + lane;
 #pragma unroll 1
-        for (int c = 0; c < p.n_tok; c += 32) {
-          if (c >= ntok) break;
+        for (int c = 32 * set; c < ntok; c += 64) {
           float v[32];
           if (t.nkb > 0) {
             pf_ld32(taddr + c, v);
@@ -472,7 +482,7 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
   }
 }
 
@@ -519,7 +529,7 @@ static int make_map(CUtensorMap* m, const void* base, int dtype, int64_t rows, i
 static int sm_pairs() { return std::max(1, num_sms() / 2); }
 
 template <typename T, int MODE>
-static int launch_pair(const PfWeightMaps& a, const CUtensorMap& b, PfArgs p, int tiles, cudaStream_t s) {
+static int launch_pair(const PfWeightMaps& a, const CUtensorMap& b, PfArgs p, int tiles, bool pdl, cudaStream_t s) {
   static bool attr_set[64] = {};
   int dev = 0;
   STX_CUDA(cudaGetDevice(&dev));
@@ -529,11 +539,17 @@ static int launch_pair(const PfWeightMaps& a, const CUtensorMap& b, PfArgs p, in
   }
   const uint32_t stage_bytes = PF_A_BYTES + static_cast<uint32_t>(p.n_tok / 2) * (PF_BK * 2);
   const uint32_t fixed = 1024 + PF_XCH_BYTES + (2 * PF_MAX_STAGES + 4) * 8 + 16;
-  p.stages = static_cast<int>(std::min<uint32_t>(PF_MAX_STAGES, (PF_SMEM - fixed) / stage_bytes));
+  // Few tokens: HBM-bound, and five or six stages per SM are enough in flight (120 KB x 148 against 6.6 TB/s x 1.5 us;
+  // four stages, which would let the next GEMM's CTA in, cost 4 %).  The rest of the shared memory is for kernels that
+  // run beside the CTA: the next layer's predictor and cache upkeep in a stack.
+  const uint32_t room = p.tok_tiles == 1 && p.n_tok <= 128 ? PF_SMEM_FEW : PF_SMEM;
+  p.stages = static_cast<int>(std::min<uint32_t>(PF_MAX_STAGES, (room - fixed) / stage_bytes));
   p.pairs = sm_pairs();
+  p.tmem_cols = 64;
+  while (p.tmem_cols < 2 * p.n_tok) p.tmem_cols *= 2;
   const size_t smem = fixed + static_cast<size_t>(p.stages) * stage_bytes;
   const unsigned grid = 2u * static_cast<unsigned>(std::max(1, std::min(tiles, p.pairs)));
-  STX_CUDA(launch_pdl(k_pair_gemm<T, MODE>, dim3(grid), dim3(PF_THREADS), smem, s, a, b, p));
+  STX_CUDA(launch_pdl_if(pdl, k_pair_gemm<T, MODE>, dim3(grid), dim3(PF_THREADS), smem, s, a, b, p));
   return STX_OK;
 }
 
@@ -586,17 +602,18 @@ bool prefill_wanted(int64_t B, int64_t H, int64_t K, int dtype, int has_gate) {
 
 template <typename T>
 static int prefill_run(const PfWeightMaps& mw, const CUtensorMap& mx, const PfArgs& g1, int tiles1, const PfWeightMaps& md,
-                       const CUtensorMap& ma, const PfArgs& g2, int tiles2, cudaStream_t s) {
-  const int rc = launch_pair<T, 0>(mw, mx, g1, tiles1, s);
-  return rc != STX_OK ? rc : launch_pair<T, 1>(md, ma, g2, tiles2, s);
+                       const CUtensorMap& ma, const PfArgs& g2, int tiles2, bool pdl, cudaStream_t s) {
+  const int rc = launch_pair<T, 0>(mw, mx, g1, tiles1, pdl, s);
+  return rc != STX_OK ? rc : launch_pair<T, 1>(md, ma, g2, tiles2, true, s);
 }
 
 // x [B,H], concat [2K,H] (gate rows then up rows), down_packed [K,H]; scratch: prefill_scratch_bytes().
 // k_dev (optional): device count of valid packed rows, <= K; the work then follows *k_dev while all
 // shapes, tensor maps and grids are built for K, so the call needs no host read-back.
+// pdl: the first kernel may overlap the end of its predecessor (no dependency on other streams).
 int prefill_forward(const void* x, int64_t B, int64_t H, const void* concat, const void* down_packed, int64_t K,
                     void* out, void* combined, int act, int dtype, void* scratch, int* status, const int* k_dev,
-                    cudaStream_t s) {
+                    bool pdl, cudaStream_t s) {
   const int64_t K8 = (K + 7) / 8 * 8;
   const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 1023) & ~static_cast<uintptr_t>(1023);
   void* a_scr = reinterpret_cast<void*>(base);                                                   // [B, K8]
@@ -645,11 +662,12 @@ int prefill_forward(const void* x, int64_t B, int64_t H, const void* concat, con
   g2.status = status;
   g2.k_dev = k_dev;
   if (s2.splits > 1) g2.part = part;
+  g2.early = 1;
   // evenly shared neurons fill all pairs even where full tiles would not
   const int tiles1 = g1.even ? sm_pairs() : static_cast<int>(w_tiles * s1.tok_tiles);
   const int tiles2 = static_cast<int>(h_tiles * s2.tok_tiles * s2.splits);
-  rc = dtype == STX_F16 ? prefill_run<__half>(mw, mx, g1, tiles1, md, ma, g2, tiles2, s)
-                        : prefill_run<__nv_bfloat16>(mw, mx, g1, tiles1, md, ma, g2, tiles2, s);
+  rc = dtype == STX_F16 ? prefill_run<__half>(mw, mx, g1, tiles1, md, ma, g2, tiles2, pdl, s)
+                        : prefill_run<__nv_bfloat16>(mw, mx, g1, tiles1, md, ma, g2, tiles2, pdl, s);
   if (rc == STX_OK && g2.part) rc = partial_sum(part, s2.splits, B * H, out, dtype, s);
   return rc;
 }
