@@ -390,6 +390,15 @@ int stx_add_rmsnorm(const void* h, const void* a, const void* w, float eps, void
 int stx_norm_gemv(const void* h, const void* a, const void* w_norm, float eps, const void* W, void* y, void* h_out,
                   void* x_out, int64_t H, int64_t N, int dtype, void* stream);
 
+/* End of a greedy decode step, one kernel: logits_out [V] = the logits in fp32, *token = the index of the largest
+ * (the first of equal ones; a NaN counts as largest, as torch.argmax has it), *pos += 1, and generated[*pos - *gen_base]
+ * = the token where that index lies in 0..max_len-1.  logits [V] in dtype; logits_out may be logits itself in fp32.
+ * workspace: 16 bytes of device memory, zeroed once by the caller and left zeroed by every call; calls that share it
+ * must be ordered on one stream.  No counterpart in the reference, whose host loop does this between forward calls
+ * (src/models/llama/modelling_llama_skip.py through transformers' generate).                  */
+int stx_decode_finish(const void* logits, int64_t V, int dtype, float* logits_out, int64_t* token, int64_t* pos,
+                      const int64_t* gen_base, int64_t* generated, int64_t max_len, void* workspace, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -78,19 +78,19 @@ template <typename T, int HD, int REP> struct AttShape {
   static constexpr int LPK = CH < 32 ? CH : 32;
   static constexpr int CPT = CH / LPK;
   static constexpr int NG = ATT_THREADS / LPK;      // rows side by side
-  static constexpr int U = (sizeof(T) == 2 && REP > 1 ? 4 : 8) / CPT;  // what 128 registers hold without spilling
+  static constexpr int U = (sizeof(T) == 4 ? 8 : REP == 1 ? 8 : REP == 4 ? 2 : 4) / CPT;  // what 128 registers hold
   static constexpr int TK = NG * U;
 };
 
 // What bounds it: the KV bytes at long contexts, a chain of dependent trips (position, rows, merge) at short ones.
 // A CTA reads every key and value of its split once for its REP query heads (they share the cache head) with 16-byte
 // loads, U keys and U values per thread requested before the first is used and the next tile's requested as soon as
-// a tile's registers are free; soft-max over tiles with a running maximum.
+// a tile's registers are free; each warp keeps a running soft-max of its own keys.
 // 24 query heads on 8 cache heads of 128, 4000 tokens, fp16: four layers of norm, attention, projection and norm 136 -> 104 us
 // (a warp per key and one batch of keys at a time before, every query head reading the cache for itself: 18.5 us a launch).
 // The splits meet in the workspace: the last one to arrive at the group's counter merges.  Splits beyond what the
 // position can use leave at once.
-// Shared memory (floats): q_s[REP][HD] | kn_s[HD] | vn_s[HD] | sc[REP][TK] | red[16][REP][HD] | m[REP] l[REP] corr[REP]
+// Shared memory (floats): q_s[REP][HD] | kn_s[HD] | vn_s[HD] | red[16][REP][HD] | m[REP][16] | l[REP][16]
 template <typename T, int HD, int REP>
 __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restrict__ qkv, const float* __restrict__ cos_t,
                                                                  const float* __restrict__ sin_t,
@@ -104,11 +104,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
   float* q_s = sm;
   float* kn_s = q_s + REP * HD;
   float* vn_s = kn_s + HD;
-  float* sc = vn_s + HD;
-  float* red = sc + REP * TK;
+  float* red = vn_s + HD;
   float* m_s = red + NW * REP * HD;
-  float* l_s = m_s + REP;
-  float* corr_s = l_s + REP;
+  float* l_s = m_s + NW * REP;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_wait();
   pdl_launch_dependents();
@@ -162,19 +160,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
   }
   __syncthreads();
 
-  // the running soft-max starts with the token's own key in the last split, with nothing in the others
-  if (warp < REP) {
-    float dot = 0.f;
-    for (int d = lane; d < HD; d += 32) dot = fmaf(q_s[warp * HD + d], kn_s[d], dot);
-    dot = warp_sum_xor(dot) * scale;
-    if (lane == 0) {
-      m_s[warp] = own ? dot : -INFINITY;
-      l_s[warp] = own ? 1.f : 0.f;
-    }
-  }
-  float qf[REP][CPT * V], acc[REP][CPT * V];
+  // Every warp runs its own soft-max over the keys that it loads (no barrier inside the loop); in the last split warp 0
+  // starts from the token's own key.
+  float qf[REP][CPT * V], acc[REP][CPT * V], m_run[REP], l_run[REP];
 #pragma unroll
-  for (int r = 0; r < REP; ++r)
+  for (int r = 0; r < REP; ++r) {
 #pragma unroll
     for (int c = 0; c < CPT; ++c)
 #pragma unroll
@@ -182,9 +172,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
         qf[r][c * V + v] = q_s[r * HD + (ch + LPK * c) * V + v];
         acc[r][c * V + v] = own && grp == 0 ? vn_s[(ch + LPK * c) * V + v] : 0.f;
       }
+    m_run[r] = -INFINITY;
+    l_run[r] = 0.f;
+    if (own && warp == 0) {
+      float dot = 0.f;
+      for (int d = lane; d < HD; d += 32) dot = fmaf(q_s[r * HD + d], kn_s[d], dot);
+      m_run[r] = warp_sum_xor(dot) * scale;
+      l_run[r] = 1.f;
+    }
+  }
 
   for (int j0 = 0; j0 < n; j0 += TK) {
-    // ---- scores of the tile
+    float p[REP][U];
 #pragma unroll
     for (int r = 0; r < REP; ++r) {
       float dot[U];
@@ -200,48 +199,33 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
         }
       }
       group_sum_many<U, LPK>(dot, lane);
-      constexpr int LPV = LPK / U;  // lanes that hold the same key's sum (LPK >= U in every instance)
-      const int u = ch / LPV;
-      if (ch % LPV == 0) sc[r * TK + grp + NG * u] = j0 + grp + NG * u < n ? dot[0] * scale : -INFINITY;
-    }
-    if (j0 + TK < n) load_tile(ks, j0 + TK, kr);
-    __syncthreads();
-    if (warp < REP) {  // a warp per query head
-      float* s = sc + warp * TK;
-      const float m_old = m_s[warp];
-      float m = m_old;
+      constexpr int LPV = LPK / U;  // lanes of a row group that hold the same key's sum (LPK >= U in every instance)
+      float mx = m_run[r];
 #pragma unroll
-      for (int i = 0; i < TK / 32; ++i) m = fmaxf(m, s[lane + 32 * i]);
+      for (int u = 0; u < U; ++u) {
+        const float s = __shfl_sync(0xffffffffu, dot[0], (lane & ~(LPK - 1)) + u * LPV) * scale;
+        p[r][u] = j0 + grp + NG * u < n ? s : -INFINITY;
+        mx = fmaxf(mx, p[r][u]);
+      }
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+      for (int off = LPK; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       float sum = 0.f;
 #pragma unroll
-      for (int i = 0; i < TK / 32; ++i) {
-        const float p = m == -INFINITY ? 0.f : __expf(s[lane + 32 * i] - m);
-        s[lane + 32 * i] = p;
-        sum += p;
+      for (int u = 0; u < U; ++u) {
+        p[r][u] = p[r][u] == -INFINITY ? 0.f : __expf(p[r][u] - mx);
+        sum += p[r][u];
       }
-      sum = warp_sum_xor(sum);
-      if (lane == 0) {
-        const float corr = m == -INFINITY ? 1.f : __expf(m_old - m);
-        m_s[warp] = m;
-        l_s[warp] = fmaf(l_s[warp], corr, sum);
-        corr_s[warp] = corr;
-      }
-    }
-    __syncthreads();
-    // ---- values of the tile
 #pragma unroll
-    for (int r = 0; r < REP; ++r) {
-      const float corr = corr_s[r];
+      for (int off = LPK; off < 32; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      const float corr = mx == m_run[r] ? 1.f : __expf(m_run[r] - mx);  // 0 where nothing came before
+      m_run[r] = mx;
+      l_run[r] = fmaf(l_run[r], corr, sum);
 #pragma unroll
       for (int k = 0; k < CPT * V; ++k) acc[r][k] *= corr;
     }
+    if (j0 + TK < n) load_tile(ks, j0 + TK, kr);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float p[REP];
-#pragma unroll
-      for (int r = 0; r < REP; ++r) p[r] = sc[r * TK + grp + NG * u];
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int c = 0; c < CPT; ++c) {
         float f[V];
@@ -249,15 +233,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
 #pragma unroll
         for (int r = 0; r < REP; ++r)
 #pragma unroll
-          for (int v = 0; v < V; ++v) acc[r][c * V + v] = fmaf(p[r], f[v], acc[r][c * V + v]);
+          for (int v = 0; v < V; ++v) acc[r][c * V + v] = fmaf(p[r][u], f[v], acc[r][c * V + v]);
       }
-    }
     if (j0 + TK < n) load_tile(vs, j0 + TK, vr);
   }
 
-  // ---- sum over the row groups: the groups of a warp by shuffle, the warps through shared memory in warp order
+  // ---- the warps' results meet in shared memory: sum_w e^(m_w - M) acc_w in warp order
 #pragma unroll
-  for (int r = 0; r < REP; ++r)
+  for (int r = 0; r < REP; ++r) {
 #pragma unroll
     for (int k = 0; k < CPT * V; ++k) {
       float a = acc[r][k];
@@ -265,23 +248,34 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
       for (int off = LPK; off < 32; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
       if (lane < LPK) red[(warp * REP + r) * HD + (ch + LPK * (k / V)) * V + k % V] = a;
     }
+    if (lane == 0) {
+      m_s[r * NW + warp] = m_run[r];
+      l_s[r * NW + warp] = l_run[r];
+    }
+  }
   __syncthreads();
   int* counter = reinterpret_cast<int*>(workspace) + blockIdx.x;
   float* part = reinterpret_cast<float*>(workspace + ATT_COUNTER_BYTES);
   auto part_of = [&](int split, int r) { return part + (static_cast<size_t>(h0 + r) * ATT_MAX_SPLITS + split) * att_part_floats(HD); };
   for (int i = tid; i < REP * HD; i += ATT_THREADS) {
     const int r = i / HD, d = i - r * HD;
-    float s = 0.f;
+    float M = -INFINITY, s = 0.f, l = 0.f;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) s += red[w * REP * HD + i];
+    for (int w = 0; w < NW; ++w) M = fmaxf(M, m_s[r * NW + w]);
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const float mw = m_s[r * NW + w], f = mw == -INFINITY ? 0.f : __expf(mw - M);  // 0 for a warp without keys
+      s = fmaf(f, red[w * REP * HD + i], s);
+      l = fmaf(f, l_s[r * NW + w], l);
+    }
     if (NSP == 1) {
-      out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(s / l_s[r]);
+      out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(s / l);
     } else {
       float* mine = part_of(sp, r);
       __stcg(mine + d, s);
       if (d == 0) {
-        __stcg(mine + HD, m_s[r]);
-        __stcg(mine + HD + 1, l_s[r]);
+        __stcg(mine + HD, M);
+        __stcg(mine + HD + 1, l);
       }
     }
   }
@@ -298,7 +292,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  float* wgt = sc;  // [REP][ATT_MAX_SPLITS] weights (TK >= 64: the scores are not needed any more)
+  float* wgt = red;  // [REP][ATT_MAX_SPLITS] weights; behind them the sums of exponentials
+  float* den_s = red + REP * ATT_MAX_SPLITS;
   if (warp < REP) {
     const float* pk = part_of(lane, warp);
     const float pm = lane < NSP ? __ldcg(pk + HD) : -INFINITY, pl = lane < NSP ? __ldcg(pk + HD + 1) : 0.f;
@@ -308,16 +303,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
     const float w = lane < NSP && pm != -INFINITY ? __expf(pm - M) : 0.f;  // 0 for a split without keys
     wgt[warp * ATT_MAX_SPLITS + lane] = w;
     const float den = warp_sum_xor(w * pl);
-    if (lane == 0) l_s[warp] = den;
+    if (lane == 0) den_s[warp] = den;
   }
   __syncthreads();
   for (int i = tid; i < REP * HD; i += ATT_THREADS) {
     const int r = i / HD, d = i - r * HD;
     const float* pk = part_of(0, r) + d;
-    float num = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < NSP; ++k) num = fmaf(wgt[r * ATT_MAX_SPLITS + k], __ldcg(pk + static_cast<size_t>(k) * att_part_floats(HD)), num);
-    out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(num / l_s[r]);
+    float v[ATT_MAX_SPLITS], num = 0.f;  // all loads in flight together
+#pragma unroll
+    for (int k = 0; k < ATT_MAX_SPLITS; ++k) v[k] = k < NSP ? __ldcg(pk + static_cast<size_t>(k) * att_part_floats(HD)) : 0.f;
+#pragma unroll
+    for (int k = 0; k < ATT_MAX_SPLITS; ++k) num = fmaf(wgt[r * ATT_MAX_SPLITS + k], v[k], num);  // weight 0 beyond NSP
+    out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(num / den_s[r]);
   }
 }
 
@@ -556,6 +553,62 @@ __global__ void __launch_bounds__(GEMV_THREADS) k_norm_gemv_tma(const T* __restr
   }
 }
 
+// Logits to fp32 and their argmax over the whole chip; the block that arrives last moves the decode state on.  A key is
+// the value in ascending unsigned order with the complemented index below it, so one 64-bit maximum finds the first of
+// the largest.  128256 fp16 logits: torch's conversion, copy, one-block argmax (30 us) and four small ops were 43 us of a
+// token, the kernel takes 5.7.
+constexpr int FIN_THREADS = 256;
+template <typename T>
+__global__ void __launch_bounds__(FIN_THREADS) k_decode_finish(const T* logits, long long V, float* logits_out, long long* token,
+                                                                long long* pos, const long long* __restrict__ gen_base,
+                                                                long long* generated, long long max_len,
+                                                                unsigned long long* __restrict__ ws) {
+  __shared__ unsigned long long s_best[FIN_THREADS / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
+  pdl_launch_dependents();
+  unsigned long long best = 0;
+  for (long long i = static_cast<long long>(blockIdx.x) * FIN_THREADS + tid; i < V; i += static_cast<long long>(gridDim.x) * FIN_THREADS) {
+    const float v = DT<T>::to_f(logits[i]);
+    logits_out[i] = v;
+    const uint32_t u = __float_as_uint(v == 0.f ? 0.f : v);  // -0 equals +0
+    const uint32_t key = v != v ? 0xffffffffu : (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+    const unsigned long long k = (static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(~static_cast<uint32_t>(i));
+    best = k > best ? k : best;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, off);
+    best = o > best ? o : best;
+  }
+  if (lane == 0) s_best[warp] = best;
+  __syncthreads();
+  if (tid != 0) return;
+#pragma unroll
+  for (int w = 1; w < FIN_THREADS / 32; ++w) best = s_best[w] > best ? s_best[w] : best;
+  atomicMax(ws, best);
+  __threadfence();
+  unsigned int* arrived = reinterpret_cast<unsigned int*>(ws + 1);
+  if (atomicAdd(arrived, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const long long t = static_cast<uint32_t>(~static_cast<uint32_t>(__ldcg(ws)));
+  *ws = 0ull;
+  *arrived = 0u;
+  const long long p = *pos + 1;
+  *pos = p;
+  *token = t;
+  const long long at = p - *gen_base;
+  if (at >= 0 && at < max_len) generated[at] = t;
+}
+template <typename T>
+static int launch_decode_finish(const void* logits, long long V, float* logits_out, long long* token, long long* pos, const long long* gen_base,
+                                long long* generated, long long max_len, void* ws, cudaStream_t s) {
+  const unsigned grid = static_cast<unsigned>(std::min<long long>(num_sms(), (V + FIN_THREADS - 1) / FIN_THREADS));
+  STX_CUDA(launch_pdl(k_decode_finish<T>, dim3(grid), dim3(FIN_THREADS), 0, s, static_cast<const T*>(logits), V, logits_out, token, pos, gen_base,
+                      generated, max_len, static_cast<unsigned long long*>(ws)));
+  return STX_OK;
+}
+
 template <typename T>
 static int launch_add_rmsnorm(const void* h, const void* a, const void* w, float eps, void* h_out, void* x_out, int H, cudaStream_t s) {
   STX_CUDA(launch_pdl(k_add_rmsnorm<T>, dim3(1), dim3(NORM_THREADS), 0, s, static_cast<const T*>(h), static_cast<const T*>(a),
@@ -600,8 +653,7 @@ static int launch_norm_gemv(const void* h, const void* a, const void* w_norm, fl
 template <typename T, int HD, int REP>
 static int launch_attn(const void* qkv, const float* cos_t, const float* sin_t, const long long* pos, void* k_cache, void* v_cache,
                        void* out, int nh, int nkv, long long max_len, float scale, void* workspace, cudaStream_t s) {
-  typedef AttShape<T, HD, REP> S;
-  constexpr int smem = static_cast<int>(sizeof(float) * ((REP + 2) * HD + REP * S::TK + ATT_THREADS / 32 * REP * HD + 3 * REP));
+  constexpr int smem = static_cast<int>(sizeof(float) * ((REP + 2) * HD + ATT_THREADS / 32 * REP * (HD + 2)));
   if (smem > 48 * 1024) {
     static bool attr_set[64] = {};
     int dev = 0;
@@ -683,6 +735,25 @@ int stx_add_rmsnorm(const void* h, const void* a, const void* w, float eps, void
     case STX_F32: return launch_add_rmsnorm<float>(h, a, w, eps, h_out, x_out, Hi, s);
     case STX_F16: return launch_add_rmsnorm<__half>(h, a, w, eps, h_out, x_out, Hi, s);
     default: return launch_add_rmsnorm<__nv_bfloat16>(h, a, w, eps, h_out, x_out, Hi, s);
+  }
+}
+
+int stx_decode_finish(const void* logits, int64_t V, int dtype, float* logits_out, int64_t* token, int64_t* pos,
+                      const int64_t* gen_base, int64_t* generated, int64_t max_len, void* workspace, void* stream) {
+  STX_CHECK_ARG(logits && logits_out && token && pos && gen_base && generated && workspace, "stx_decode_finish: null pointer");
+  STX_CHECK_ARG(V > 0 && V <= 0x7fffffff, "stx_decode_finish: V=%lld out of range", static_cast<long long>(V));
+  STX_CHECK_ARG(dtype == STX_F32 || dtype == STX_F16 || dtype == STX_BF16, "stx_decode_finish: bad dtype %d", dtype);
+  STX_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 7) == 0, "stx_decode_finish: workspace must be 8-byte aligned");
+  static_assert(sizeof(int64_t) == sizeof(long long), "token and position types");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  long long* t = reinterpret_cast<long long*>(token);
+  long long* p = reinterpret_cast<long long*>(pos);
+  const long long* g = reinterpret_cast<const long long*>(gen_base);
+  long long* out = reinterpret_cast<long long*>(generated);
+  switch (dtype) {
+    case STX_F32: return launch_decode_finish<float>(logits, V, logits_out, t, p, g, out, max_len, workspace, s);
+    case STX_F16: return launch_decode_finish<__half>(logits, V, logits_out, t, p, g, out, max_len, workspace, s);
+    default: return launch_decode_finish<__nv_bfloat16>(logits, V, logits_out, t, p, g, out, max_len, workspace, s);
   }
 }
 

@@ -107,6 +107,14 @@ def attn_decode(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: to
     return out
 
 
+def decode_finish(logits: torch.Tensor, logits_out: torch.Tensor, token: torch.Tensor, pos: torch.Tensor, gen_base: torch.Tensor,
+                  generated: torch.Tensor, workspace: torch.Tensor) -> None:
+    """logits_out <- logits in fp32, token[0] <- their argmax, pos[0] += 1, generated[pos[0] - gen_base[0]] <- token[0]."""
+    C.check(C.lib.stx_decode_finish(logits.data_ptr(), logits.numel(), _DT[logits.dtype], logits_out.data_ptr(), token.data_ptr(),
+                                    pos.data_ptr(), gen_base.data_ptr(), generated.data_ptr(), generated.numel(),
+                                    workspace.data_ptr(), torch.cuda.current_stream().cuda_stream))
+
+
 def rope_tables(cfg: LlamaSkipConfig, device) -> tuple[torch.Tensor, torch.Tensor]:
     inv = 1.0 / (cfg.rope_theta ** (torch.arange(0, cfg.head_dim, 2, device=device, dtype=torch.float32) / cfg.head_dim))
     ang = torch.arange(cfg.max_len, device=device, dtype=torch.float32)[:, None] * inv[None, :]
@@ -156,6 +164,7 @@ class LlamaSkipModel:
         self._side = torch.cuda.Stream(device=self.device)    # cache index plans
         self._side2 = torch.cuda.Stream(device=self.device)   # cache row copies
         self._attn_ws = attn_workspace(cfg.heads, cfg.head_dim, self.device)
+        self._finish_ws = torch.zeros(16, dtype=torch.uint8, device=self.device)
         self._graph = None
         self.trace = None  # when a list: per decode step and layer (x_pred, x_mlp, mlp_out, mask) copies, eager mode only
 
@@ -230,11 +239,7 @@ class LlamaSkipModel:
         return out
 
     def _finish_token(self, last: torch.Tensor) -> None:
-        self.logits.copy_((last @ self.embed.t()).float().view(-1))
-        nxt = self.logits.argmax().view(1)
-        self.pos.add_(1)
-        self.token.copy_(nxt)
-        self.generated.index_copy_(0, self.pos - self.gen_base, nxt)
+        decode_finish(last @ self.embed.t(), self.logits, self.token, self.pos, self.gen_base, self.generated, self._finish_ws)
 
     def _decode_body_native(self) -> None:
         cfg = self.cfg
