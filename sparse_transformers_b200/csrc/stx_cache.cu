@@ -18,14 +18,37 @@
 
 namespace stx {
 
+// 32 mask bytes (non-zero = active) as one word; neurons from I on are off.
+__device__ __forceinline__ uint32_t mask_word_of_bytes(const uint8_t* __restrict__ bytes, int w, int I) {
+  const uint8_t* p = bytes + static_cast<size_t>(w) * 32;
+  uint32_t word = 0u;
+  if (w * 32 + 32 <= I && (reinterpret_cast<uintptr_t>(bytes) & 15) == 0) {
+    const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
+    const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int q = 0; q < 8; ++q)  // bytes -> 0/1 bytes -> four neighbouring bits (byte i moves from bit 8 i to bit 24 + i)
+      word |= (((__vcmpne4(v[q], 0u) & 0x01010101u) * 0x01020408u) >> 24 & 0xfu) << (4 * q);
+  } else {
+    for (int i = 0; i < 32 && w * 32 + i < I; ++i) word |= static_cast<uint32_t>(p[i] != 0) << i;
+  }
+  return word;
+}
+
+// The new mask as bits, or (BYTES) as one byte per neuron, packed on the way in.
+template <bool BYTES>
 __global__ void __launch_bounds__(PLAN_THREADS, 1)
-k_cache_plan(const uint32_t* __restrict__ new_bits, uint32_t* __restrict__ cur_bits,
+k_cache_plan(const void* __restrict__ mask, uint32_t* __restrict__ cur_bits,
              int32_t* __restrict__ active, int32_t* __restrict__ pos_of, int32_t* __restrict__ lists,
              int32_t* __restrict__ jobs, int32_t* __restrict__ state, uint32_t* __restrict__ stale, int lazy, int I) {
   extern __shared__ int32_t sm[];
   pdl_wait();
   pdl_launch_dependents();
-  plan_block(new_bits, cur_bits, active, pos_of, lists, jobs, state, stale, lazy, I, sm);
+  plan_block(
+      [&](int w) {
+        if constexpr (BYTES) return mask_word_of_bytes(static_cast<const uint8_t*>(mask), w, I);
+        else return static_cast<const uint32_t*>(mask)[w];
+      },
+      cur_bits, active, pos_of, lists, jobs, state, stale, lazy, I, sm);
 }
 
 // One warp per (job, matrix): packed[m][pos] = pool[m][active[pos]], 16-byte vectors.
@@ -107,23 +130,25 @@ __global__ void k_fill_i32(int32_t* p, int32_t v, size_t n) {
 
 static size_t plan_smem_bytes(int64_t I) { return plan_smem_words(I) * sizeof(int32_t); }
 
-int cache_plan(stx_cache* c, const uint32_t* bits, cudaStream_t s, bool lazy, bool pdl) {
+template <bool BYTES>
+static int launch_plan(stx_cache* c, const void* mask, cudaStream_t s, bool lazy, bool pdl) {
   static bool attr_set[64] = {};
   int dev = 0;
   STX_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    STX_CUDA(cudaFuncSetAttribute(k_cache_plan, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    STX_CUDA(cudaFuncSetAttribute(k_cache_plan<BYTES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(plan_smem_bytes(MAX_I))));
     attr_set[dev] = true;
   }
   // two mask words per thread at most; small index spaces use fewer threads (cheaper barriers)
   const int W = static_cast<int>((c->I + 31) / 32);
   const int threads = W <= 256 ? 256 : (W <= 512 ? 512 : PLAN_THREADS);
-  STX_CUDA(launch_pdl_if(pdl, k_cache_plan, dim3(1), dim3(threads), plan_smem_bytes(c->I), s, bits, c->cur_bits, c->active, c->pos_of,
+  STX_CUDA(launch_pdl_if(pdl, k_cache_plan<BYTES>, dim3(1), dim3(threads), plan_smem_bytes(c->I), s, mask, c->cur_bits, c->active, c->pos_of,
                          c->lists, c->jobs, c->state, c->stale, lazy ? 1 : 0, static_cast<int>(c->I)));
   if (lazy) c->lazy_used = true;
   return STX_OK;
 }
+int cache_plan(stx_cache* c, const uint32_t* bits, cudaStream_t s, bool lazy, bool pdl) { return launch_plan<false>(c, bits, s, lazy, pdl); }
 
 // Turns the stale bitmap into the job list (slots below K, ascending) and clears it.
 __global__ void __launch_bounds__(1024, 1)
@@ -179,13 +204,15 @@ int cache_copy_rows(stx_cache* c, cudaStream_t s, bool pdl) {
   return STX_OK;
 }
 
-int cache_update_bits(stx_cache* c, const uint32_t* bits, cudaStream_t s) {
+template <bool BYTES>
+static int cache_update(stx_cache* c, const void* mask, cudaStream_t s) {
   int rc = cache_flush(c, s);  // rows left stale by earlier lazy plans come first
   if (rc != STX_OK) return rc;
-  rc = cache_plan(c, bits, s, false, true);
+  rc = launch_plan<BYTES>(c, mask, s, false, true);
   if (rc != STX_OK) return rc;
   return cache_copy_rows(c, s, true);
 }
+int cache_update_bits(stx_cache* c, const uint32_t* bits, cudaStream_t s) { return cache_update<false>(c, bits, s); }
 
 // cat[n] = [gate[n] | up[n] | down[n]] (nmat rows of vec 16-byte vectors each)
 __global__ void __launch_bounds__(256)
@@ -222,8 +249,14 @@ int cache_ensure_cat(stx_cache* c, cudaStream_t s) {
   return STX_OK;
 }
 
+// A store to the pinned mirror instead of a copy: no hand-over between the compute and the copy engine.
+__global__ void k_state_to_host(const int32_t* state, int32_t* host) {
+  pdl_wait();
+  if (threadIdx.x < ST_COUNT) host[threadIdx.x] = state[threadIdx.x];
+}
+
 int cache_read_state(stx_cache* c, cudaStream_t s) {
-  STX_CUDA(cudaMemcpyAsync(c->host_state, c->state, ST_COUNT * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  STX_CUDA(launch_pdl(k_state_to_host, dim3(1), dim3(32), 0, s, c->state, c->host_state));
   STX_CUDA(cudaStreamSynchronize(s));
   return STX_OK;
 }
@@ -264,7 +297,6 @@ int stx_cache_destroy(stx_cache_t* c) {
   cudaFree(c->lists);
   cudaFree(c->jobs);
   cudaFree(c->cur_bits);
-  cudaFree(c->tmp_bits);
   cudaFree(c->stale);
   cudaFree(c->state);
   if (c->host_state) cudaFreeHost(c->host_state);
@@ -341,7 +373,6 @@ int stx_cache_create(stx_cache_t** out, int64_t I, int64_t H, int dtype, int has
   STX_ALLOC(c->lists, 2 * I * sizeof(int32_t));
   STX_ALLOC(c->jobs, I * sizeof(int32_t));
   STX_ALLOC(c->cur_bits, W * sizeof(uint32_t));
-  STX_ALLOC(c->tmp_bits, W * sizeof(uint32_t));
   STX_ALLOC(c->stale, W * sizeof(uint32_t));
   STX_ALLOC(c->state, ST_COUNT * sizeof(int32_t));
   if (cudaMallocHost(reinterpret_cast<void**>(&c->host_state), ST_COUNT * sizeof(int32_t)) != cudaSuccess) {
@@ -414,9 +445,7 @@ int stx_mask_bits_to_bytes(const uint32_t* bits, int64_t I, uint8_t* bytes_out, 
 
 int stx_cache_update(stx_cache_t* c, const uint8_t* mask_bytes, void* stream) {
   STX_CHECK_ARG(c && mask_bytes, "stx_cache_update: null argument");
-  int rc = stx_mask_bytes_to_bits(mask_bytes, c->I, c->tmp_bits, stream);
-  if (rc != STX_OK) return rc;
-  return cache_update_bits(c, c->tmp_bits, static_cast<cudaStream_t>(stream));
+  return cache_update<true>(c, mask_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int stx_cache_update_bits(stx_cache_t* c, const uint32_t* mask_bits, void* stream) {

@@ -48,7 +48,6 @@ struct stx_cache {
   int32_t* lists = nullptr;    // [2I] scratch: added ids | removed ids (ascending)
   int32_t* jobs = nullptr;     // [I] packed positions to rewrite from the pool
   uint32_t* cur_bits = nullptr;  // [W] current mask
-  uint32_t* tmp_bits = nullptr;  // [W] staging for byte masks
   uint32_t* stale = nullptr;     // [W] packed slots whose rows lag behind the index plan (lazy mode)
   bool lazy_used = false;        // host flag: some plan was enqueued (or captured) in lazy mode
   int32_t* state = nullptr;      // [ST_COUNT]

@@ -63,7 +63,9 @@ __device__ __forceinline__ Int2 block_excl_scan2(Int2 v, Int2* total, Int2* warp
 // lists in global memory.
 // All threads of the block call it (blockDim.x a multiple of 32, at most 2 mask words per thread); `sm` is the
 // block's work space of plan_smem_words(I) words.  Ends without a block barrier.
-__device__ __forceinline__ void plan_block(const uint32_t* __restrict__ new_bits, uint32_t* __restrict__ cur_bits,
+// new_word(w): word w of the new mask, called once per word.
+template <typename NewWord>
+__device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restrict__ cur_bits,
                                            int32_t* __restrict__ active, int32_t* __restrict__ pos_of, int32_t* __restrict__ lists,
                                            int32_t* __restrict__ jobs, int32_t* __restrict__ state, uint32_t* __restrict__ stale, int lazy,
                                            int I, int32_t* sm) {
@@ -91,7 +93,7 @@ __device__ __forceinline__ void plan_block(const uint32_t* __restrict__ new_bits
   for (int k = 0; k < WPT; ++k) {
     const int w = t * WPT + k;
     if (w < W) {
-      uint32_t nb = new_bits[w];
+      uint32_t nb = new_word(w);
       const uint32_t ob = cur_bits[w];
       if (w == W - 1 && (I & 31)) nb &= (1u << (I & 31)) - 1u;
       nbw[k] = nb;

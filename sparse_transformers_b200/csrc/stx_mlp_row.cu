@@ -814,7 +814,7 @@ __device__ __forceinline__ bool plan_in_last_block(const PlanCall& pc) {
   if constexpr (PLAN) {
     extern __shared__ int32_t plan_sm[];
     if (blockIdx.x == gridDim.x - 1) {
-      plan_block(pc.bits, pc.u.cur_bits, pc.u.active, pc.u.pos_of, pc.u.lists, pc.u.jobs, pc.u.state, pc.u.stale, pc.u.lazy, pc.I, plan_sm);
+      plan_block([&](int w) { return pc.bits[w]; }, pc.u.cur_bits, pc.u.active, pc.u.pos_of, pc.u.lists, pc.u.jobs, pc.u.state, pc.u.stale, pc.u.lazy, pc.I, plan_sm);
       return true;
     }
   }

@@ -504,7 +504,8 @@ __global__ void __launch_bounds__(SB1_THREADS, 1) k_stack_flow(const __grid_cons
   if (q.upkeep != nullptr && c < L) {
     __syncthreads();  // every thread is done with the slots
     const UpkeepArgs* ua = q.upkeep + c;
-    plan_block(q.layer[c].bits, ua->cur_bits, ua->active, ua->pos_of, ua->lists, ua->jobs, ua->state, ua->stale, ua->lazy, I,
+    const uint32_t* new_bits = q.layer[c].bits;
+    plan_block([&](int w) { return new_bits[w]; }, ua->cur_bits, ua->active, ua->pos_of, ua->lists, ua->jobs, ua->state, ua->stale, ua->lazy, I,
                reinterpret_cast<int32_t*>(slots));
     // the plan's work space becomes row buffers of phase C, which bulk copies write through the async proxy
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
