@@ -165,9 +165,11 @@ struct PfWeightMaps {
   CUtensorMap m[4];
 };
 
-// Box of at least `rows` rows: 1 + its index in PfWeightMaps, 0 for none.  A box may fetch rows beyond the CTA's share
-// (its neighbour's, on their way through the L2 anyway); their products land in accumulator lanes that nobody reads.
-__device__ __forceinline__ int pf_box(int rows) { return rows > 32 ? 1 : rows > 16 ? 2 : rows > 8 ? 3 : rows > 0 ? 4 : 0; }
+// Box (index in PfWeightMaps) of at least `rows` rows.  It may fetch rows beyond the CTA's share (its neighbour's, on
+// their way through the L2 anyway); their products land in accumulator lanes that nobody reads.  A CTA without rows
+// fetches eight as well: every producer has a part in every stage, so the ring can never run past one of them (a
+// producer that nothing waits for can fall two uses of a stage behind, where the parity of its barrier reads as pending).
+__device__ __forceinline__ int pf_box(int rows) { return rows > 32 ? 0 : rows > 16 ? 1 : rows > 8 ? 2 : 3; }
 
 // One tile of a pair's walk.
 struct PfTile {
@@ -284,7 +286,7 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
   }
 
   const uint32_t full0 = pf_mapa(full, 0);  // the even CTA's barriers
-  const int k_valid = p.k_dev ? min(*p.k_dev, MODE == 0 ? p.N : p.Kd) : (MODE == 0 ? p.N : p.Kd);
+  const int k_valid = p.k_dev ? min(__ldcg(p.k_dev), MODE == 0 ? p.N : p.Kd) : (MODE == 0 ? p.N : p.Kd);
   const PfPlan plan = pf_plan<MODE>(p, k_valid);
   bool timed_out = false;
 
@@ -297,13 +299,12 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
       for (int it = pair; it < plan.tiles && !timed_out; it += npairs) {
         const PfTile t = pf_tile<MODE>(plan, it);
         const int box0 = pf_box(t.m_rows0), box1 = pf_box(t.m_rows1);
-        const uint32_t bytes = (MODE == 0 ? ((box0 ? 64u >> (box0 - 1) : 0u) + (box1 ? 64u >> (box1 - 1) : 0u)) * (2 * PF_BK * 2) : 2 * PF_A_BYTES) + 2 * b_bytes;
+        const uint32_t bytes = (MODE == 0 ? ((64u >> box0) + (64u >> box1)) * (2 * PF_BK * 2) : 2 * PF_A_BYTES) + 2 * b_bytes;
         const int box = rank ? box1 : box0;
         const int m0 = MODE == 0 ? t.m0 + (rank ? t.m_rows0 : 0) + (part == 1 ? p.N : 0)
                                  : t.m0 + static_cast<int>(rank) * 128 + part * 64;
         const int tok = t.tok0 + static_cast<int>(rank) * (p.n_tok / 2);
-        const CUtensorMap* map = part == 2 ? &tmB : &tmA.m[MODE == 0 && box > 1 ? box - 1 : 0];
-        const bool issue = part == 2 || MODE == 1 || box > 0;
+        const CUtensorMap* map = part == 2 ? &tmB : &tmA.m[MODE == 0 ? box : 0];
         // One token tile: all pairs stream weights at once, and rows of a power of two of bytes would have every one of
         // them ask for the same columns at the same time; each starts at another k block instead (GEMM 1 of 64 tokens,
         // 8700 neurons of 4096: 44.4 -> 41.5 us)
@@ -315,11 +316,9 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
           }
           unsigned char* dst = smem + static_cast<size_t>(s) * stage_bytes + (part == 2 ? PF_A_BYTES : part * 8192u);
           if (rank == 0 && part == 0) pf_expect_tx(&full[s], bytes);
-          if (issue) {
-            if (part == 2) pf_tma_2d(dst, map, k, tok, full0 + s * 8);
-            else if (MODE == 0) pf_tma_2d(dst, map, k, m0, full0 + s * 8);
-            else pf_tma_2d(dst, map, m0, k, full0 + s * 8);
-          }
+          if (part == 2) pf_tma_2d(dst, map, k, tok, full0 + s * 8);
+          else if (MODE == 0) pf_tma_2d(dst, map, k, m0, full0 + s * 8);
+          else pf_tma_2d(dst, map, m0, k, full0 + s * 8);
           k += PF_BK;
           if (MODE == 0 && k >= t.nkb * PF_BK) k = 0;
           if (++s == S) {
@@ -475,6 +474,7 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
       }
     }
   }
+  __syncwarp();  // the producing lanes are back: what follows is executed by whole warps
   if (timed_out && p.status && lane == 0) atomicOr(p.status, DEV_TIMEOUT);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

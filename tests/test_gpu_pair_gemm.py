@@ -39,6 +39,27 @@ def test_against_torch_fp32(dtype, B, H, K, act):
     assert bool(((out.double() - ref).abs() <= eps * ref.abs() + 1e-4 * ref.abs().max()).all())
 
 
+@pytest.mark.parametrize("K", [1000, 1016, 8704 + 64])
+def test_a_last_tile_for_one_cta_of_the_pair(K):
+    """The last tile has eight neurons, all of the even CTA's: no wait of the odd one may run out (each costs about a second)."""
+    from stxgpu import DEV, mlp_forward
+
+    H, B = 4096, 64
+    g = torch.Generator(device=DEV).manual_seed(K)
+    rn = lambda *s: (torch.randn(*s, generator=g, device=DEV) / 64).to(torch.bfloat16)
+    x, cw, dp = rn(B, H), rn(2 * K, H), rn(K, H)
+    first = None
+    for _ in range(150):
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        out, _ = mlp_forward(x, cw, dp, "silu")
+        t1.record()
+        t1.synchronize()
+        assert t0.elapsed_time(t1) < 300.0
+        first = out if first is None else first
+        assert torch.equal(out, first)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("B,H,r,I,density", [
     (9, 4096, 32, 100, 0.1),      # smallest row block
