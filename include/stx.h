@@ -297,7 +297,9 @@ int stx_layer_step_host(stx_layer_t* l, const void* x_host, int64_t B, void* out
  *   STX_STACK_KERNEL=layers   keep the per-layer kernels (k_pred_t, k_mlp_b1, k_partial_reduce)
  *   STX_STACK_GROUP=n         at most n layers per launch of the persistent kernel (1..36)
  * Other shapes and batch sizes: the per-layer kernels, serialised on one stream, each layer's
- * cache upkeep on side branches.                                                         */
+ * cache upkeep on side branches.  Row blocks (9 rows and more, 16-bit, gated) with all stages
+ * and distinct layers and caches: predictors and cache upkeep of all layers on two branches of
+ * the graph, ahead of the layers' GEMMs, since they need the stack's input only.            */
 int stx_stack_create(stx_stack_t** out, stx_layer_t* const* layers, int64_t L, int64_t B);
 /* Same, capturing only the given STX_STAGE_* bits of every layer step.                  */
 int stx_stack_create_stages(stx_stack_t** out, stx_layer_t* const* layers, int64_t L, int64_t B,
