@@ -202,7 +202,7 @@ static bool single_row_fusable(const stx_layer* l, int64_t B) {
 // Up to 8 rows under a rule that needs whole score rows (top-k, statistical): the same kernels with the finished mask
 // instead of their own scores.  One row: k_mlp_b1 on the listed bits, as the general path would, but with the index
 // plan next to the sum.  2..8 rows (16-bit gated weights): k_mlp_bn.  Against the gate/up and down kernels of the general
-// path (which it replaces there): 3 rows of 4096 x 11008, 10 % per row, 107 -> 59 us a
+// path (which it replaces there): 3 rows of 4096 x 11008, 10 % per row, 107 -> 60 us a
 // step together with the selection kernel of stx_select.cu (30 -> 10 us).
 static bool given_mask_fusable(const stx_layer* l, int64_t B) {
   const stx_cache* c = l->cache;

@@ -413,10 +413,8 @@ __global__ void __launch_bounds__(512, 1) k_mlp_b1(const MlpB1Args q) {
 //                batch rows, k = the (up to) 8 neurons of the tile (m16n8k8).  Warp w owns columns
 //                w*H/16 .. and keeps its H/16 x 8 outputs in registers; the A fragments come
 //                transposed out of the down rows with ldmatrix.trans; a is rounded to the model
-//                dtype for the B fragment (as the reference's own activations are).  GIVEN: a goes in
-//                as the sum of two numbers of the model dtype, a = hi + lo, with m16n8k16: k 0..7
-//                multiply hi and k 8..15 lo with the same A registers (16 or 22 mantissa bits); an
-//                fp16 tile whose largest |a| is out of range is scaled by a power of two meanwhile.
+//                dtype for the B fragment (as the reference's own activations are).  GIVEN: a stays in
+//                fp32, so the product runs on the FMA pipe (see k_mlp_bn).
 // A buffer is re-filled with the next tile's rows as soon as its phase is over, so two of the three
 // are in flight or ready while the third is being read.  Filling all 16 tile rows matters: the
 // kernel's instruction stream is dominated by the fragment loads of x (64 KB per tile pass) and the
@@ -439,15 +437,25 @@ constexpr uint32_t BN_POLL_LIMIT = 1u << 20;
 constexpr int BN_MAX = 8;
 constexpr int BN_TN_MAX = 8;
 constexpr int BN_MT_MAX = 16;  // m-tiles of 16 columns per warp: H <= 16 * 16 * 16
-constexpr int BN_HEADER = 1024;                // [0,64) 3 mbarriers | [256,512) a: hi, then lo, [4 neuron pairs][8 rows of the batch]
+constexpr int BN_PAIRS = 4;    // pairs of columns per thread (GIVEN): H <= 2 * 512 * 4
+// [0,64) 3 mbarriers | [256,512) a of a tile: in the model dtype [4 neuron pairs][8 rows of the batch], or fp32 [8 neurons][8 rows]
+constexpr int BN_HEADER = 1024;
 constexpr int BN_RED_BYTES = 16 * 16 * 8 * 4;  // [warp][tile row][batch] fp32
 
-// Power of two that brings activations of up to `amax` into the range of fp16 (1 where they fit, and for infinities and NaN).
-__device__ __forceinline__ float bn_scale(float amax) {
-  return amax > 32768.f && amax < INFINITY ? exp2f(static_cast<float>(14 - ilogbf(amax))) : 1.f;
+// Two neighbouring 16-bit weights.
+template <typename T>
+__device__ __forceinline__ float2 unpack_pair(uint32_t w) {
+  if constexpr (DT<T>::id == STX_BF16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  else return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
 
-// GIVEN: the mask is finished (q.bits) and a keeps the accuracy of fp32, as in the kernels this variant stands in for.
+// GIVEN: the mask is finished (q.bits) and a stays in fp32 through the down projection, as in the kernels this variant
+// stands in for: the weights are converted, and a thread adds up two neighbouring columns of every 1024, all rows, with
+// FMAs.  So a row of the batch owes nothing to its neighbours, and no activation is too small or too large for the model
+// dtype.  As two numbers of the model dtype on the tensor pipe, a would lose bits below 2^-3 in fp16 (16 bits are all it
+// has in bf16) and need a scale per row; four tokens at 10 % per row, 4096 x 11008 fp16, take 239 us at 3 rows and 333 at
+// 8 here, 237 and 332 there (2048 x 11008 bf16, 8 rows: 254 and 239; the separate kernels: 426, 704 and 481).  Pairs of
+// columns in fma.rn.f32x2 are slower (240, 340 and 251): they need a twice per row from shared memory.
 // Leaving registers for the row copies of the layer before (120 instead of 128 here, 32 in k_cache_copy_rows), so that
 // they run beside this kernel and not between two launches of it, was built and is slower: the copies take from the rows
 // that the CTAs wait for (8 layers of 4096 x 14336, 8 rows: 607 against 543 us a token).
@@ -469,8 +477,8 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
   uint64_t* bar_x = reinterpret_cast<uint64_t*>(smem);
   uint64_t* bar_y = bar_x + 1;
   uint64_t* bar_z = bar_x + 2;
-  uint32_t* a_pk = reinterpret_cast<uint32_t*>(smem + 256);  // [hi, lo][neuron pair][batch row]: (a[2k][b], a[2k+1][b]) in the model dtype
-  __shared__ float s_amax[2];
+  uint32_t* a_pk = reinterpret_cast<uint32_t*>(smem + 256);  // [neuron pair][batch row]: (a[2k][b], a[2k+1][b]) in the model dtype
+  float* a_s = reinterpret_cast<float*>(smem + 256);         // GIVEN: [neuron][batch row]
   const size_t t_bytes = pred_t_smem_bytes(B, q.r, V);
   float* t_s = reinterpret_cast<float*>(smem + BN_HEADER);
   float* red_s = reinterpret_cast<float*>(smem + BN_HEADER + t_bytes);
@@ -545,7 +553,7 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
     fill(0, 0);
     fill(1, 0);
   }
-  if (early && niter > 0 && nlocal < TN) {
+  if (!GIVEN && early && niter > 0 && nlocal < TN) {
     // a short only tile: the unused down rows are multiplied by a = 0, so they must hold finite numbers
     for (int i = tid; i < TN * static_cast<int>(zstride / 16); i += blockDim.x)
       reinterpret_cast<uint4*>(Z)[i] = make_uint4(0, 0, 0, 0);
@@ -648,7 +656,7 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
     if (blockIdx.x == 0 && tid == 0) *reinterpret_cast<volatile int*>(xc) = epoch;
     __syncthreads();
     if (!early) {
-      if (niter > 0 && nlocal < TN) {  // as above: unused down rows must hold finite numbers
+      if (!GIVEN && niter > 0 && nlocal < TN) {  // as above: unused down rows must hold finite numbers
         for (int i = tid; i < TN * static_cast<int>(zstride / 16); i += blockDim.x)
           reinterpret_cast<uint4*>(Z)[i] = make_uint4(0, 0, 0, 0);
         __syncthreads();
@@ -667,6 +675,12 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) dacc[mt][k] = 0.f;
   const int MT = H / 256;  // m-tiles per warp (even)
+  // GIVEN: outputs of this thread, columns 1024 c + 2 tid and the next one of every row
+  float2 oacc[BN_PAIRS][BN_MAX];
+#pragma unroll
+  for (int c = 0; c < BN_PAIRS; ++c)
+#pragma unroll
+    for (int b = 0; b < BN_MAX; ++b) oacc[c][b] = make_float2(0.f, 0.f);
 
   const int nwh = H / 64;  // windows (32 consecutive k = 64 bytes) per half row
   const int w_lo = (nwh * warp) / 16, w_hi = (nwh * (warp + 1)) / 16;  // this warp's share of each half
@@ -716,34 +730,38 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
         a = apply_act(p.act, g) * u;
       }
       if constexpr (GIVEN) {
-        if (DT<T>::id == STX_F16) {
-          float m = fabsf(a);
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-          if (lane == 0) s_amax[warp] = m;
-          asm volatile("bar.sync 1, 64;" ::: "memory");
-          a *= bn_scale(fmaxf(s_amax[0], s_amax[1]));
-        }
-        const float hi = DT<T>::round_f(a);
-        const float lo = isinf(hi) ? 0.f : a - hi;
-        const float hi_next = __shfl_down_sync(0xffffffffu, hi, 8);  // neuron e + 1, same batch row
-        const float lo_next = __shfl_down_sync(0xffffffffu, lo, 8);
-        if ((e & 1) == 0) {
-          a_pk[(e >> 1) * 8 + b] = MmaK8<T>::pack(hi, hi_next);
-          a_pk[32 + (e >> 1) * 8 + b] = MmaK8<T>::pack(lo, lo_next);
-        }
+        a_s[tid] = a;
       } else {
         const float a_next = __shfl_down_sync(0xffffffffu, a, 8);  // neuron e + 1, same batch row
         if ((e & 1) == 0) a_pk[(e >> 1) * 8 + b] = MmaK8<T>::pack(a, a_next);
       }
     }
-    __syncthreads();  // a_pk complete
+    __syncthreads();  // the activations are complete
     // ---- phase 2
     if (!mbar_wait_bounded(bar_z, parity)) timed_out = true;
-    {
-      const uint32_t bfrag = a_pk[tq * 8 + gq];                     // B[k = 2tq, 2tq+1][n = gq]
-      const uint32_t blo = GIVEN ? a_pk[32 + tq * 8 + gq] : 0u;     // B[k = 2tq + 8, 2tq + 9][n = gq]
-      const float scale = GIVEN && DT<T>::id == STX_F16 ? bn_scale(fmaxf(s_amax[0], s_amax[1])) : 1.f;
+    if constexpr (GIVEN) {
+#pragma unroll 2
+      for (int e = 0; e < nv; ++e) {
+        const float4 a03 = *reinterpret_cast<const float4*>(a_s + e * BN_MAX);
+        const float4 a47 = *reinterpret_cast<const float4*>(a_s + e * BN_MAX + 4);
+        const float av[BN_MAX] = {a03.x, a03.y, a03.z, a03.w, a47.x, a47.y, a47.z, a47.w};
+        const unsigned char* zrow = Z + static_cast<size_t>(e) * zstride + tid * 4;
+#pragma unroll
+        for (int c = 0; c < BN_PAIRS; ++c) {
+          if (c * 512 + tid < H / 2) {
+            const float2 w = unpack_pair<T>(*reinterpret_cast<const uint32_t*>(zrow + c * 2048));
+#pragma unroll
+            for (int b = 0; b < BN_MAX; ++b) {
+              if (b < 4 || B > 4) {
+                oacc[c][b].x = fmaf(av[b], w.x, oacc[c][b].x);
+                oacc[c][b].y = fmaf(av[b], w.y, oacc[c][b].y);
+              }
+            }
+          }
+        }
+      }
+    } else {
+      const uint32_t bfrag = a_pk[tq * 8 + gq];  // B[k = 2tq, 2tq+1][n = gq]
       // ldmatrix row of this lane: neuron lane & 7 (a missing row of a short buffer reads row 0, its a is 0),
       // 8-column group lane >> 3 of the 32 columns of an m-tile pair
       const int zr = (lane & 7) < TN ? (lane & 7) : 0;
@@ -753,32 +771,29 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
         if (2 * mp < MT) {
           uint32_t af[4];
           ldmatrix_x4_trans(af, zrow + static_cast<size_t>(mp) * 64);
-          if constexpr (!GIVEN) {
-            MmaK8<T>::run(dacc[2 * mp], af[0], af[1], bfrag);
-            MmaK8<T>::run(dacc[2 * mp + 1], af[2], af[3], bfrag);
-          } else if (DT<T>::id == STX_F16 && scale != 1.f) {
-            float t0[4] = {0.f, 0.f, 0.f, 0.f}, t1[4] = {0.f, 0.f, 0.f, 0.f};
-            MmaOp<T>::run16(t0, af[0], af[1], af[0], af[1], bfrag, blo);
-            MmaOp<T>::run16(t1, af[2], af[3], af[2], af[3], bfrag, blo);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              dacc[2 * mp][k] += t0[k] / scale;
-              dacc[2 * mp + 1][k] += t1[k] / scale;
-            }
-          } else {
-            MmaOp<T>::run16(dacc[2 * mp], af[0], af[1], af[0], af[1], bfrag, blo);
-            MmaOp<T>::run16(dacc[2 * mp + 1], af[2], af[3], af[2], af[3], bfrag, blo);
-          }
+          MmaK8<T>::run(dacc[2 * mp], af[0], af[1], bfrag);
+          MmaK8<T>::run(dacc[2 * mp + 1], af[2], af[3], bfrag);
         }
       }
     }
     if (it + 1 < niter) {
-      __syncthreads();  // every thread is done with a_pk and the down rows of this tile
+      __syncthreads();  // every thread is done with the activations and the down rows of this tile
       fill(2, it + 1);
     }
   }
   if (timed_out && p.status) atomicOr(p.status, DEV_TIMEOUT);
-  {
+  if constexpr (GIVEN) {
+    float* dst = q.partial + static_cast<size_t>(blockIdx.x) * B * H + 2 * tid;
+#pragma unroll
+    for (int b = 0; b < BN_MAX; ++b) {
+      if (b < B) {
+#pragma unroll
+        for (int c = 0; c < BN_PAIRS; ++c)
+          if (c * 512 + tid < H / 2)
+            *reinterpret_cast<float2*>(dst + static_cast<size_t>(b) * H + c * 1024) = oacc[c][b];
+      }
+    }
+  } else {
     float* dst = q.partial + static_cast<size_t>(blockIdx.x) * B * H + static_cast<size_t>(warp) * (H / 16) + gq;
     const int b0 = 2 * tq, b1 = 2 * tq + 1;
 #pragma unroll

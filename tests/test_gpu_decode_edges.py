@@ -95,6 +95,45 @@ def test_finished_masks_through_the_layer(rule, param, B, dtype, scale):
             assert float(a.abs().max()) > 65504
 
 
+def _mlp_terms(x, gate, up, down, on):
+    """act(g) * u of the active neurons in 64 bits, the result, and the size of its terms (what the sums' rounding scales with)."""
+    a = torch.nn.functional.silu(x.double() @ gate[on].double().t()) * (x.double() @ up[on].double().t())
+    d = down[:, on].double().t()
+    return a, a @ d, a.abs() @ d.abs()
+
+
+@pytest.mark.parametrize("dtype,H,I,k,scales,wd", [
+    (torch.float16, 4096, 6000, 900, (12000.0, 1.0, 0.1, 0.03), 0.05),   # 20 and more neurons a CTA: several tiles of six
+    (torch.float16, 512, 3000, 2500, (3e-3, 3e-3), 1.0),                 # activations around 1e-6, tiles of eight
+    (torch.float16, 1024, 4736, 1500, (1.0,) * 8, 0.05),
+    (torch.bfloat16, 2048, 6000, 1200, (1e4, 1.0, 1e-4), 0.05),
+    (torch.bfloat16, 512, 200, 3, (1.0, 1.0, 1.0, 1.0, 1.0), 0.05),      # fewer neurons than CTAs
+])
+def test_finished_masks_keep_rows_apart_and_fp32_activations(dtype, H, I, k, scales, wd):
+    from sparse_transformers_b200 import SparseLayer
+
+    B, r = len(scales), 32
+    g = torch.Generator(device=DEV).manual_seed(H + k)
+    rn = lambda *s, std=1.0: (torch.randn(*s, generator=g, device=DEV) * std).to(dtype)
+    gate, up, down = rn(I, H, std=0.02), rn(I, H, std=0.02), rn(H, I, std=wd)
+    layer = SparseLayer(gate, up, down, rn(r, H, std=0.02), rn(I, r, std=0.02), act="silu", method="topk", param=k, max_batch=B)
+    fi = torch.finfo(dtype)
+    for _ in range(2):
+        x_pred = rn(B, H)
+        x = (x_pred.float() * torch.tensor(scales, device=DEV)[:, None]).to(dtype)
+        out = layer.step(x_pred, x)
+        on = layer.mask()
+        _, ref, size = _mlp_terms(x, gate, up, down, on)
+        # one rounding of the result (half a step of the smallest numbers at least); fp32 sums of H and of K terms
+        bound = fi.eps * ref.abs() + fi.smallest_normal * fi.eps + 2e-5 * size
+        fits = ref.abs() < 0.99 * fi.max
+        assert bool(((out.double() - ref).abs() <= bound)[fits].all())
+        for other in (0.0, float("inf"), float("nan")):  # what stands in row 0 is nothing to the other rows
+            x2 = x.clone()
+            x2[0] = other
+            assert torch.equal(layer.step(x_pred, x2)[1:], out[1:]), other
+
+
 @pytest.mark.parametrize("B", [2, 8, 12, 70])
 def test_stack_with_predictors_ahead_equals_eager_layers(B):
     from sparse_transformers_b200 import SparseLayer, SparseStack
