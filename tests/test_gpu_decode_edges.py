@@ -160,3 +160,40 @@ def test_stack_with_predictors_ahead_equals_eager_layers(B):
     two = torch.empty(2, B, H, dtype=dt, device=DEV)
     both.step(x, two)
     assert torch.equal(two[0], out[0]) and torch.equal(two[1], out[0])
+
+
+@pytest.mark.parametrize("H,I", [(512, 2048), (4096, 8192), (8192, 9000)])
+def test_norm_gemv_waits_for_the_kernel_that_writes_its_weights(H, I):
+    """The row copies of a cache update let the next kernel of the stream start before they are through."""
+    import ctypes
+
+    from stxgpu import Cache, stream
+
+    from sparse_transformers_b200 import _capi as C
+    from sparse_transformers_b200.llama_skip import norm_gemv
+
+    dt = torch.float16
+    g = torch.Generator(device=DEV).manual_seed(H)
+    up = (torch.randn(I, H, generator=g, device=DEV) * 0.02).to(dt)
+    cache = Cache(up, up, up.t().contiguous())
+    pk = ctypes.c_void_p()
+    C.check(C.lib.stx_cache_packed_ptrs(cache.h, None, ctypes.byref(pk), None, None))
+    h, a, wn = (torch.randn(1, H, generator=g, device=DEV).to(dt) for _ in range(3))
+    masks = [torch.arange(I, device=DEV) % 2 == i for i in (0, 1)]
+    K = int(masks[0].sum())
+    masks[1][: K - int(masks[1].sum())] = True  # as many in both
+
+    class Packed:
+        __cuda_array_interface__ = {"shape": (K * H * 2,), "typestr": "|u1", "data": (pk.value, False), "version": 2}
+
+    W = torch.as_tensor(Packed(), device=DEV).view(dt).view(K, H)
+    own = torch.empty(K, H, dtype=dt, device=DEV)
+    for it in range(12):
+        C.check(C.lib.stx_cache_update(cache.h, masks[it % 2].data_ptr(), stream()))
+        first = norm_gemv(h, None, None, 0.0, W) if it % 3 else norm_gemv(h, a, wn, 1e-5, W)
+        torch.cuda.synchronize()
+        assert torch.equal(first, norm_gemv(h, None, None, 0.0, W) if it % 3 else norm_gemv(h, a, wn, 1e-5, W))
+        torch.mul(W, float(it + 1), out=own)  # a torch kernel in front
+        first = norm_gemv(h, None, None, 0.0, own)
+        torch.cuda.synchronize()
+        assert torch.equal(first, norm_gemv(h, None, None, 0.0, own))
