@@ -409,6 +409,9 @@ int stx_cache_create(stx_cache_t** out, int64_t I, int64_t H, int dtype, int has
   if (e == cudaSuccess) e = cudaMemsetAsync(c->state, 0, ST_COUNT * sizeof(int32_t), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(c->pos_of, 0xff, I * sizeof(int32_t), s);  // -1
   if (e == cudaSuccess) e = cudaMemsetAsync(c->active, 0xff, I * sizeof(int32_t), s);
+  // row blocks (16-bit, gated) multiply the packed down rows in whole blocks of 64: those behind the last active row meet
+  // activations of zero, so they must hold numbers
+  if (e == cudaSuccess && has_gate && es == 2) e = cudaMemsetAsync(c->pk_down, 0, mat, s);
   if (e != cudaSuccess) {
     int rc = cuda_fail(e, "stx_cache_create: initialisation");
     stx_cache_destroy(c);

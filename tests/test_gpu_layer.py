@@ -214,3 +214,30 @@ def test_two_to_eight_rows_one_kernel_path(B, dtype, act, H, I):
     assert probe.single_row_fused(B)
     probe.close()
     _run(w, steps=6, seed=11)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B", [12, 200])
+def test_row_block_on_a_cache_that_starts_empty(dtype, B):
+    """The packed rows behind the last active one are no neuron's: their memory may hold anything."""
+    from sparse_transformers_b200 import SparseLayer
+    from stxgpu import DEV, Cache
+
+    H, I, r, k = 512, 1000, 32, 70
+    g = torch.Generator(device=DEV).manual_seed(B)
+    rn = lambda *s, std=1.0: (torch.randn(*s, generator=g, device=DEV) * std).to(dtype)
+    gate, up, down = rn(I, H, std=0.05), rn(I, H, std=0.05), rn(H, I, std=0.05)
+    nan = torch.full((I, H), float("nan"), dtype=dtype, device=DEV)
+    for _ in range(2):  # leaves the allocator blocks of these sizes full of NaN
+        Cache(nan, nan, nan.t().contiguous()).close()
+        torch.cuda.synchronize()
+        layer = SparseLayer(gate, up, down, rn(r, H), rn(I, r), act="silu", method="topk", param=k, max_batch=B, init_all_active=False)
+        x = rn(1, H).expand(B, H).contiguous()  # equal rows: exactly k active neurons, 70 of two blocks of 64
+        out = layer.step(x).double()
+        on = layer.mask()
+        assert int(on.sum()) == k
+        a = (torch.nn.functional.silu(x.double() @ gate[on].double().t()) * (x.double() @ up[on].double().t())).to(dtype).double()
+        ref = a @ down[:, on].double().t()
+        eps = torch.finfo(dtype).eps  # a rounding of the activations (and fp32 sums) and one of the result
+        assert bool(((out - ref).abs() <= eps * ref.abs() + eps * (a.abs() @ down[:, on].double().abs().t())).all())
+        layer.close()
