@@ -182,7 +182,10 @@ k_stale_to_jobs(uint32_t* __restrict__ stale, int32_t* __restrict__ jobs, int32_
       d &= d - 1;
     }
   }
-  if (t == 0) state[ST_NJOBS] = s_tot.x;
+  if (t == 0) {
+    state[ST_NJOBS] = s_tot.x;
+    state[ST_STALE] = 0;
+  }
 }
 
 // Brings the packed rows up to date after lazy plans.  A cache that has ever been planned

@@ -12,6 +12,7 @@ enum : int {
   ST_STATUS = 4,   // stx::DEV_* bits (sticky)
   ST_VALID = 5,    // 1 once an update has rebuilt the views (reference: cache_valid)
   ST_EPOCH = 6,    // incremented by every update that changed something
+  ST_STALE = 7,    // 1 while the stale bitmap may have bits
   ST_COUNT = 8
 };
 

@@ -64,6 +64,8 @@ __device__ __forceinline__ Int2 block_excl_scan2(Int2 v, Int2* total, Int2* warp
 // All threads of the block call it (blockDim.x a multiple of 32, at most 2 mask words per thread); `sm` is the
 // block's work space of plan_smem_words(I) words.  Ends without a block barrier.
 // new_word(w): word w of the new mask, called once per word.
+// lazy: the rewritten slots are remembered in `stale` and no job is listed.  Otherwise the slots that earlier lazy plans
+// left in `stale` join this plan's jobs, so a caller that copies the listed rows leaves no row behind.
 template <typename NewWord>
 __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restrict__ cur_bits,
                                            int32_t* __restrict__ active, int32_t* __restrict__ pos_of, int32_t* __restrict__ lists,
@@ -88,6 +90,7 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
 
   // ---- 1. diff words (weight_cache.h:84-110: added = new & ~old, removed = old & ~new)
   const int K0 = state[ST_K];
+  const bool fold = !lazy && state[ST_STALE] != 0;
   uint32_t nbw[2] = {0, 0}, aw[2] = {0, 0}, rw[2] = {0, 0};
   Int2 cnt{0, 0};
   for (int k = 0; k < WPT; ++k) {
@@ -105,11 +108,20 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
       cnt.y += __popc(rw[k]);
     }
   }
+  if (fold) {
+    for (int k = 0; k < WPT; ++k) {
+      const int w = t * WPT + k;
+      if (w < W) {
+        s_dirty[w] = stale[w];
+        stale[w] = 0u;
+      }
+    }
+  }
   if (t == 0) s_slow = 0;
   Int2 off = block_excl_scan2(cnt, &s_tot, s_ws);
   const int na = s_tot.x, nr = s_tot.y;
 
-  if (na == 0 && nr == 0) {  // unchanged mask: the reference returns before touching anything
+  if (na == 0 && nr == 0 && !fold) {  // unchanged mask: the reference returns before touching anything
     if (t == 0) {
       state[ST_NJOBS] = 0;
       state[ST_ADDED] = 0;
@@ -319,6 +331,8 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
     }
   }
   if (t == 0) {
+    if (lazy) state[ST_STALE] = 1;
+    else if (fold) state[ST_STALE] = 0;
     state[ST_K] = Knew;
     state[ST_ADDED] = na;
     state[ST_REMOVED] = nr;

@@ -241,3 +241,41 @@ def test_row_block_on_a_cache_that_starts_empty(dtype, B):
         eps = torch.finfo(dtype).eps  # a rounding of the activations (and fp32 sums) and one of the result
         assert bool(((out - ref).abs() <= eps * ref.abs() + eps * (a.abs() @ down[:, on].double().abs().t())).all())
         layer.close()
+
+
+@pytest.mark.parametrize("stack", [False, True])
+@pytest.mark.parametrize("method,param", [("naive", None), ("topk", 300)])
+def test_row_block_after_lazy_steps(stack, method, param):
+    """Rows that lazy steps have left behind are brought up to date before a row block multiplies them."""
+    from sparse_transformers_b200 import SparseLayer, SparseStack
+    from stxgpu import DEV
+
+    H, I, r, B, dt = 512, 1030, 32, 16, torch.float16
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rn = lambda *s, std=1.0: (torch.randn(*s, generator=g, device=DEV) * std).to(dt)
+    w = (rn(I, H, std=0.05), rn(I, H, std=0.05), rn(H, I, std=0.05), rn(r, H, std=0.02), rn(I, r, std=0.02))
+    param = 0.02 ** 2 * np.sqrt(H * r) * 0.8 if param is None else param
+    lazy, eager = (SparseLayer(*w, act="silu", method=method, param=param, max_batch=B, lazy_cache=z) for z in (True, False))
+    block = SparseStack([lazy], B) if stack else None
+    out = torch.empty(1, B, H, dtype=dt, device=DEV)
+
+    def both(x):
+        want = eager.step(x)
+        if block is not None and x.shape[0] == B:
+            block.step(x, out)
+            assert torch.equal(out[0], want)
+        else:
+            assert torch.equal(lazy.step(x), want)
+        assert torch.equal(lazy.mask(), eager.mask())
+
+    for _ in range(3):
+        for _ in range(3):
+            both(rn(1, H))
+        both(rn(B, H))
+        x = rn(1, H)
+        both(x)
+        both(x.expand(B, H).contiguous())  # the mask of the lazy step before: nothing changes but the rows
+        both(rn(3, H))
+        both(rn(B, H))
+    assert torch.equal(lazy.concat_weight(), eager.concat_weight())
+    assert lazy.active_indices().tolist() == eager.active_indices().tolist()
