@@ -90,7 +90,7 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
 
   // ---- 1. diff words (weight_cache.h:84-110: added = new & ~old, removed = old & ~new)
   const int K0 = state[ST_K];
-  const bool fold = !lazy && state[ST_STALE] != 0;
+  const int behind = state[ST_STALE];
   uint32_t nbw[2] = {0, 0}, aw[2] = {0, 0}, rw[2] = {0, 0};
   Int2 cnt{0, 0};
   for (int k = 0; k < WPT; ++k) {
@@ -108,18 +108,10 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
       cnt.y += __popc(rw[k]);
     }
   }
-  if (fold) {
-    for (int k = 0; k < WPT; ++k) {
-      const int w = t * WPT + k;
-      if (w < W) {
-        s_dirty[w] = stale[w];
-        stale[w] = 0u;
-      }
-    }
-  }
   if (t == 0) s_slow = 0;
   Int2 off = block_excl_scan2(cnt, &s_tot, s_ws);
   const int na = s_tot.x, nr = s_tot.y;
+  const bool fold = !lazy && behind != 0;  // looked at behind the scan, where its load has long come back
 
   if (na == 0 && nr == 0 && !fold) {  // unchanged mask: the reference returns before touching anything
     if (t == 0) {
@@ -140,6 +132,11 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
   for (int k = 0; k < WPT; ++k) {
     const int w = t * WPT + k;
     if (w < W) {
+      if (fold) {
+        s_dirty[w] = stale[w];
+        stale[w] = 0u;
+        state[ST_STALE] = 0;
+      }
       s_remoff[w] = off.y;
       uint32_t a = aw[k], r = rw[k];
       while (a) {
@@ -302,7 +299,10 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
     if (w < W) {
       uint32_t d = s_dirty[w];
       if (lazy) {
-        if (d) stale[w] |= d;
+        if (d) {
+          stale[w] |= d;
+          state[ST_STALE] = 1;
+        }
         d = 0u;
       }
       const int lo = w * 32;
@@ -331,8 +331,6 @@ __device__ __forceinline__ void plan_block(NewWord new_word, uint32_t* __restric
     }
   }
   if (t == 0) {
-    if (lazy) state[ST_STALE] = 1;
-    else if (fold) state[ST_STALE] = 0;
     state[ST_K] = Knew;
     state[ST_ADDED] = na;
     state[ST_REMOVED] = nr;
