@@ -863,7 +863,7 @@ def prefill_measure(args, dev):
             "roofline": {"kernel": "k_pair_gemm", "bound": "tensor", "achieved": top["tflops"], "peak": peak,
                          "unit": "TFLOP/s", "frac": top["tflops"] / peak, "peak_source": peak_src, "traffic": None,
                          "flops_per_step": 6.0 * T * H * I},
-            "k_sweep": sweep, "gpu_launches": 3 * steps,
+            "k_sweep": sweep, "gpu_launches": 2 * steps,  # the two GEMMs; at this many rows neither is split
             "l2": "x (64 MB) + packed weights (270 MB at K = I) exceed the 126 MB L2"}
 
 

@@ -605,11 +605,11 @@ __global__ void __launch_bounds__(FIN_THREADS) k_decode_finish(const T* logits, 
   if (at >= 0 && at < max_len) generated[at] = t;
 }
 template <typename T>
-static int launch_decode_finish(const void* logits, long long V, float* logits_out, long long* token, long long* pos, const long long* gen_base,
-                                long long* generated, long long max_len, void* ws, cudaStream_t s) {
+static int launch_decode_finish(const void* logits, long long V, float* logits_out, long long* token, long long* pos,
+                                const long long* gen_base, long long* generated, long long max_len, void* ws, cudaStream_t s) {
   const unsigned grid = static_cast<unsigned>(std::min<long long>(num_sms(), (V + FIN_THREADS - 1) / FIN_THREADS));
-  STX_CUDA(launch_pdl(k_decode_finish<T>, dim3(grid), dim3(FIN_THREADS), 0, s, static_cast<const T*>(logits), V, logits_out, token, pos, gen_base,
-                      generated, max_len, static_cast<unsigned long long*>(ws)));
+  STX_CUDA(launch_pdl(k_decode_finish<T>, dim3(grid), dim3(FIN_THREADS), 0, s, static_cast<const T*>(logits), V, logits_out,
+                      token, pos, gen_base, generated, max_len, static_cast<unsigned long long*>(ws)));
   return STX_OK;
 }
 

@@ -470,8 +470,9 @@ static int capture_status(stx_stack* s, cudaStream_t cs) {
 }
 
 // A stack of row blocks: the predictor and the cache upkeep of a layer need the stack's input only, not the layer
-// before, so they run on two branches of their own (predictors; upkeep), ahead of the GEMMs, which leave them shared
-// memory and registers on every SM.  Layers that share an object (or a cache) stay serial.
+// before, so they run on two branches of their own (predictors; upkeep), ahead of the GEMMs.  Up to 128 rows those leave
+// them shared memory and registers on every SM; larger blocks fill the SMs, and the branches take turns with them.
+// Layers that share an object (or a cache) stay serial.
 static bool row_blocks_ahead(const stx_stack* s, unsigned stages) {
   if (stages != STX_STAGE_ALL) return false;
   for (size_t i = 0; i < s->layers.size(); ++i) {

@@ -817,8 +817,10 @@ __global__ void __launch_bounds__(512, 1) k_mlp_bn(const MlpB1Args q) {
 // (pa.world > 1: the layer is one shard of several GPUs) the column sums are then exchanged
 // over peer memory and added in rank order before the output is written: the all-reduce of the
 // sharded down projection costs no extra launch.
-// PLAN: one more block, the last, runs the index plan of the layer's cache (one row of 2048 x 8192 in fp32: 42 -> 37 us a step): the plan needs the mask only, which is as old as
-// the partial vectors, and takes about as long as the sum.
+// PLAN: one more block, the last, runs the index plan of the layer's cache: the plan needs the mask only, which is as old
+// as the partial vectors.  It saves a launch (one row of 2048 x 8190 in fp16 without a gate, statistical rule: 38 -> 29 us
+// a step together with the dependent launches of plan and copies; one row of 2048 x 8192 in fp32: 40 -> 36, of which runs
+// of the same code differ by as much) and outlasts the sum by some us, so it is the end of the step's chain.
 struct PlanCall {
   const uint32_t* bits;
   UpkeepArgs u;
@@ -829,7 +831,8 @@ __device__ __forceinline__ bool plan_in_last_block(const PlanCall& pc) {
   if constexpr (PLAN) {
     extern __shared__ int32_t plan_sm[];
     if (blockIdx.x == gridDim.x - 1) {
-      plan_block([&](int w) { return pc.bits[w]; }, pc.u.cur_bits, pc.u.active, pc.u.pos_of, pc.u.lists, pc.u.jobs, pc.u.state, pc.u.stale, pc.u.lazy, pc.I, plan_sm);
+      plan_block([&](int w) { return pc.bits[w]; }, pc.u.cur_bits, pc.u.active, pc.u.pos_of, pc.u.lists, pc.u.jobs,
+                 pc.u.state, pc.u.stale, pc.u.lazy, pc.I, plan_sm);
       return true;
     }
   }
@@ -967,7 +970,8 @@ struct B1Pred {  // predictor back half fused into k_mlp_b1 (Bm == nullptr: not 
 // Sum of the CTAs' partial vectors (four columns per thread with `wide`), with the cache's index plan in one more block
 // where the caller asks for it.
 template <typename T, bool PLAN>
-static int launch_reduce_plan(const float* partial, int G, int n, bool wide, void* out, const B1Pred& pr, const PlanCall& pc, cudaStream_t s) {
+static int launch_reduce_plan(const float* partial, int G, int n, bool wide, void* out, const B1Pred& pr, const PlanCall& pc,
+                              cudaStream_t s) {
   const size_t smem = PLAN ? plan_smem_words(pc.I) * sizeof(int32_t) : 0;
   if (PLAN) {
     static bool attr_set[64] = {};
@@ -1137,31 +1141,19 @@ __global__ void __launch_bounds__(256) k_partial_sum_few(const float* __restrict
 }
 
 // out[i] = sum over g < G of partial[g][i] in ascending g (n a multiple of 128), model dtype.
-int partial_sum(const float* partial, int G, int64_t n, void* out, int dtype, cudaStream_t s) {
-  STX_CHECK_ARG(n % 128 == 0 && n / 128 < (1ll << 31), "partial_sum: n must be a multiple of 128");
-  if (G <= 16) {
-    const int nn = static_cast<int>(n);
-    const dim3 grid(static_cast<unsigned>((n / 4 + 255) / 256));
-    switch (dtype) {
-      case STX_F32: STX_CUDA(launch_pdl(k_partial_sum_few<float>, grid, dim3(256), 0, s, partial, G, nn, static_cast<float*>(out))); break;
-      case STX_F16: STX_CUDA(launch_pdl(k_partial_sum_few<__half>, grid, dim3(256), 0, s, partial, G, nn, static_cast<__half*>(out))); break;
-      default:
-        STX_CUDA(launch_pdl(k_partial_sum_few<__nv_bfloat16>, grid, dim3(256), 0, s, partial, G, nn, static_cast<__nv_bfloat16*>(out)));
-        break;
-    }
-    return STX_OK;
-  }
-  const PeerArgs none = {};
-  const int nn = static_cast<int>(n);
-  switch (dtype) {
-    case STX_F32: STX_CUDA(launch_pdl(k_partial_reduce4<float, false>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn, static_cast<float*>(out), none, PlanCall{})); break;
-    case STX_F16: STX_CUDA(launch_pdl(k_partial_reduce4<__half, false>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn, static_cast<__half*>(out), none, PlanCall{})); break;
-    default:
-      STX_CUDA(launch_pdl(k_partial_reduce4<__nv_bfloat16, false>, dim3(nn / 128), dim3(1024), 0, s, partial, G, nn,
-                          static_cast<__nv_bfloat16*>(out), none, PlanCall{}));
-      break;
-  }
+template <typename T>
+static int launch_partial_sum(const float* partial, int G, int64_t n, void* out, cudaStream_t s) {
+  STX_CUDA(launch_pdl(k_partial_sum_few<T>, dim3(static_cast<unsigned>((n / 4 + 255) / 256)), dim3(256), 0, s, partial, G,
+                      static_cast<int>(n), static_cast<T*>(out)));
   return STX_OK;
+}
+int partial_sum(const float* partial, int G, int64_t n, void* out, int dtype, cudaStream_t s) {
+  STX_CHECK_ARG(n % 128 == 0 && n < (1ll << 31), "partial_sum: n must be a multiple of 128, below 2^31");
+  switch (dtype) {
+    case STX_F32: return launch_partial_sum<float>(partial, G, n, out, s);
+    case STX_F16: return launch_partial_sum<__half>(partial, G, n, out, s);
+    default: return launch_partial_sum<__nv_bfloat16>(partial, G, n, out, s);
+  }
 }
 
 bool layer_b1_supported(int64_t B, int64_t H, int64_t I, int64_t r, int has_gate, int dtype, const void* gate,

@@ -535,8 +535,8 @@ static int launch_scores_mma(const float* t_scratch, const void* Bm, uint32_t* b
   const int64_t W = (I + 31) / 32;
   const int64_t tile = std::min<int64_t>(B, PSM_ROWS);
   const size_t smem = static_cast<size_t>((tile + 7) / 8 * 8) * (r + 8) * sizeof(T);
-  STX_CUDA(launch_pdl(k_pred_scores_mma<T>, dim3(static_cast<unsigned>((W + PSM_WARPS - 1) / PSM_WARPS), static_cast<unsigned>((B + tile - 1) / tile)),
-                      dim3(PSM_WARPS * 32), smem, s, t_scratch, static_cast<const T*>(Bm), bits, static_cast<int>(B),
+  const dim3 grid(static_cast<unsigned>((W + PSM_WARPS - 1) / PSM_WARPS), static_cast<unsigned>((B + tile - 1) / tile));
+  STX_CUDA(launch_pdl(k_pred_scores_mma<T>, grid, dim3(PSM_WARPS * 32), smem, s, t_scratch, static_cast<const T*>(Bm), bits, static_cast<int>(B),
                       static_cast<int>(tile), static_cast<int>(r), static_cast<int>(I), tau, merge));
   return STX_OK;
 }
@@ -646,9 +646,7 @@ extern "C" {
 
 int stx_predict_scratch_bytes(int64_t B, int64_t I, int64_t r, size_t* bytes_out) {
   STX_CHECK_ARG(bytes_out && B > 0 && I > 0 && r > 0, "stx_predict_scratch_bytes: bad argument");
-  // t [B,r] fp32, then per-row selection scratch (B x 4 floats + B x ceil(I/32) words)
-  *bytes_out = align_up(static_cast<size_t>(B) * r * sizeof(float), 256) +
-               align_up(static_cast<size_t>(B) * (16 + ((I + 31) / 32) * sizeof(uint32_t)), 256);
+  *bytes_out = align_up(static_cast<size_t>(B) * r * sizeof(float), 256);  // t [B,r] fp32
   return STX_OK;
 }
 

@@ -21,12 +21,13 @@
 //   warps 0, 6, 7  producers: TMA tiled loads (128-byte swizzle) of a 64-wide k block per stage, one
 //               box of the stage each (gate / up rows or the two column boxes / tokens): a warp
 //               issues about one box per 85 ns, and three in a row made the issue the bottleneck
-//               (64 tokens, 8700 neurons of 4096: GEMM 1 57 -> 44 us).  Both CTAs' copies complete on the even CTA's barrier
+//               (64 tokens, 8700 neurons of 4096: GEMM 1 57 -> 44 us).  Both CTAs' copies complete on the
+//               even CTA's barrier
 //   warp 1      even CTA: issues the MMAs from one lane; tcgen05.commit (multicast to both CTAs)
 //               releases a stage / publishes an accumulator.  Allocates and frees tensor memory.
 //   warps 2..5 and 8..11  epilogue, every other 32 tokens each: tcgen05.ld 32 lanes x 32 tokens; a
-//               warp's 32 lanes are neighbouring columns of the result, so every store is one contiguous 64- or 128-byte piece
-//               whatever the alignment of the row.
+//               warp's 32 lanes are neighbouring columns of the result, so every store is one contiguous
+//               64- or 128-byte piece whatever the alignment of the row.
 // Edges are handled by TMA zero fill on loads and by masked stores; no load is multicast.
 // Every mbarrier wait is bounded; a role whose wait expired records DEV_TIMEOUT, stops, and the
 // others run out of their own waits in turn, so that TMEM is always freed.
@@ -238,8 +239,9 @@ __device__ __forceinline__ PfTile pf_tile(const PfPlan& q, int it) {
   return t;
 }
 
-// tmA[i]: weights, box 64 k x (64 >> i) rows (MODE 0) / [0] only, 64 columns x 64 k rows (MODE 1); tmB: tokens, box 64 x n_tok/2.  Dynamic shared memory (1024-byte aligned): stages x (A tile | token tile),
-// exchange buffers of the epilogue, then full[S], empty[S], acc_full[2], acc_empty[2], TMEM base address.
+// tmA[i]: weights, box 64 k x (64 >> i) rows (MODE 0) / [0] only, 64 columns x 64 k rows (MODE 1); tmB: tokens, box
+// 64 x n_tok/2.  Dynamic shared memory (1024-byte aligned): stages x (A tile | token tile), exchange buffers of the
+// epilogue, then full[S], empty[S], acc_full[2], acc_empty[2], TMEM base address.
 template <typename T, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PF_THREADS, 1)
 k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CUtensorMap tmB, const PfArgs p) {
@@ -272,7 +274,8 @@ k_pair_gemm(const __grid_constant__ PfWeightMaps tmA, const __grid_constant__ CU
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // tensor memory: this warp of both CTAs allocates, the same warps free
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pf_smem(tmem_slot)), "r"(p.tmem_cols) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pf_smem(tmem_slot)), "r"(p.tmem_cols)
+                 : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -573,7 +576,8 @@ static PfShape pair_shape(int64_t B, int64_t m_tiles, int64_t nkb, int64_t H, bo
     for (int64_t z = 1; z <= (may_split ? 16 : 1); ++z) {
       if (z > 1 && (z * B > PF_SPLIT_ROWS || z > nkb)) break;
       const double tiles = static_cast<double>(m_tiles * tiles_t * z), pairs = sm_pairs();
-      const double waves = even && tiles_t == 1 ? tiles / pairs : static_cast<double>((m_tiles * tiles_t * z + sm_pairs() - 1) / sm_pairs());
+      const double waves =
+          even && tiles_t == 1 ? tiles / pairs : static_cast<double>((m_tiles * tiles_t * z + sm_pairs() - 1) / sm_pairs());
       double t = waves * static_cast<double>((nkb + z - 1) / z) * kb_us;
       if (z > 1) t += 3.0 + 8.0 * static_cast<double>(z * B * H) / 5e6;
       if (t < best_t * 0.999) {

@@ -129,7 +129,7 @@ __device__ __forceinline__ uint32_t block_kth_largest(KeyAt key_at, int n, int k
 
 template <typename T>
 __global__ void __launch_bounds__(SEL_THREADS)
-k_mask_statistical(const T* __restrict__ scores, int I, float z, uint32_t* __restrict__ bits, float* __restrict__ cutoff_out) {
+k_mask_statistical(const T* __restrict__ scores, int I, float z, uint32_t* __restrict__ bits) {
   __shared__ double s_w[32];
   __shared__ double s_out;
   const T* s = scores + static_cast<size_t>(blockIdx.x) * I;
@@ -151,7 +151,6 @@ k_mask_statistical(const T* __restrict__ scores, int I, float z, uint32_t* __res
   const float z_r = DT<T>::round_f(z);
   const float prod = DT<T>::round_f(__fmul_rn(std_r, z_r));
   const float cutoff = DT<T>::round_f(__fadd_rn(mean_r, prod));
-  if (t == 0 && cutoff_out) cutoff_out[blockIdx.x] = cutoff;
   const int W = (I + 31) >> 5, lane = t & 31;
   for (int w = t >> 5; w < W; w += SEL_THREADS / 32) {
     const int i = w * 32 + lane;
@@ -293,12 +292,18 @@ int mask_from_scores(const void* scores, int64_t B, int64_t I, int dtype, int me
   if (!zeroed) STX_CUDA(cudaMemsetAsync(bits_out, 0, W * sizeof(uint32_t), s));
   const dim3 grid(static_cast<unsigned>(B)), block(SEL_THREADS);
   const int ii = static_cast<int>(I);
-  float* no_cutoff = nullptr;
   if (method == STX_MASK_STATISTICAL) {
     switch (dtype) {
-      case STX_F32: STX_CUDA(launch_pdl(k_mask_statistical<float>, grid, block, 0, s, static_cast<const float*>(scores), ii, param, bits_out, no_cutoff)); break;
-      case STX_F16: STX_CUDA(launch_pdl(k_mask_statistical<__half>, grid, block, 0, s, static_cast<const __half*>(scores), ii, param, bits_out, no_cutoff)); break;
-      default: STX_CUDA(launch_pdl(k_mask_statistical<__nv_bfloat16>, grid, block, 0, s, static_cast<const __nv_bfloat16*>(scores), ii, param, bits_out, no_cutoff)); break;
+      case STX_F32:
+        STX_CUDA(launch_pdl(k_mask_statistical<float>, grid, block, 0, s, static_cast<const float*>(scores), ii, param, bits_out));
+        break;
+      case STX_F16:
+        STX_CUDA(launch_pdl(k_mask_statistical<__half>, grid, block, 0, s, static_cast<const __half*>(scores), ii, param, bits_out));
+        break;
+      default:
+        STX_CUDA(launch_pdl(k_mask_statistical<__nv_bfloat16>, grid, block, 0, s, static_cast<const __nv_bfloat16*>(scores), ii,
+                            param, bits_out));
+        break;
     }
     return STX_OK;
   }
