@@ -42,7 +42,10 @@ __device__ __forceinline__ float block_reduce(float v, float* red) {
 // split the unnormalised value sum [HD], the split's score maximum and its sum of exponentials.
 constexpr size_t ATT_COUNTER_BYTES = 4096;  // up to 1024 heads
 constexpr int ATT_MAX_SPLITS = 32;
-constexpr int ATT_KEYS_PER_SPLIT = 48;      // a split of fewer keys costs more in the merge than it saves
+// One block takes up to ATT_TILES_ALONE tiles of keys by itself, beyond that a split takes at least ATT_KEYS_PER_SPLIT: a
+// second tile costs a block 0.5 to 1 us, the merge of splits 1.5 to 2.5 us whatever their number.
+constexpr int ATT_TILES_ALONE = 2;
+constexpr int ATT_KEYS_PER_SPLIT = 48;
 __host__ __device__ inline int att_part_floats(int hd) { return hd + 2; }
 
 // Sums of v[0..N) over groups of G neighbouring lanes (powers of two).  A stage halves the values a lane keeps, as long
@@ -89,7 +92,11 @@ template <typename T, int HD, int REP> struct AttShape {
 // 24 query heads on 8 cache heads of 128, 4000 tokens, fp16: four layers of norm, attention, projection and norm 136 -> 104.5 us
 // (a warp per key and one batch of keys at a time before, every query head reading the cache for itself: 18.5 us a launch).
 // The splits meet in the workspace: the last one to arrive at the group's counter merges.  Splits beyond what the
-// position can use leave at once.
+// position can use leave at once.  Between 64 and 1000 keys the ends of the chain are what counts: the warps' sums in
+// lane order (no bank conflicts) with their weights formed once, one release per block instead of a fence per thread, and
+// partial sums requested together with their weights took the same four layers from 78 to 74 us at 200 keys and from 103
+// to 98 at 4000 (32 heads on 8: 103 to 97 and 126 to 116; before the heads of a cache head shared a block: 74 and 135,
+// 96 and 167).
 // Shared memory (floats): q_s[REP][HD] | kn_s[HD] | vn_s[HD] | red[16][REP][HD] | m[REP][16] | l[REP][16]
 template <typename T, int HD, int REP>
 __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restrict__ qkv, const float* __restrict__ cos_t,
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
   if (pos < 0 || pos >= max_len) return;  // nothing sensible to do; the output is left as it was
   const int h0 = blockIdx.x * REP, g = h0 / (nh / nkv);
   const int np = static_cast<int>(pos);   // cached keys
-  const int NSP = min(static_cast<int>(gridDim.y), np / ATT_KEYS_PER_SPLIT + 1);
+  const int NSP = np <= ATT_TILES_ALONE * TK ? 1 : min(static_cast<int>(gridDim.y), np / ATT_KEYS_PER_SPLIT + 1);
   const int sp = blockIdx.y;
   if (sp >= NSP) return;
   T* kc = k_cache + static_cast<size_t>(g) * max_len * HD;
@@ -238,7 +245,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
     if (j0 + TK < n) load_tile(vs, j0 + TK, vr);
   }
 
-  // ---- the warps' results meet in shared memory: sum_w e^(m_w - M) acc_w in warp order
+  // ---- the warps' results meet in shared memory: sum_w e^(m_w - M) acc_w in warp order.  Until the result is written, a
+  // row's elements stand in the order of the lanes that hold them (element `slot` = k * LPK + ch), so that neighbouring
+  // lanes touch neighbouring banks.
 #pragma unroll
   for (int r = 0; r < REP; ++r) {
 #pragma unroll
@@ -246,52 +255,79 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
       float a = acc[r][k];
 #pragma unroll
       for (int off = LPK; off < 32; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-      if (lane < LPK) red[(warp * REP + r) * HD + (ch + LPK * (k / V)) * V + k % V] = a;
+      if (lane < LPK) red[(warp * REP + r) * HD + k * LPK + lane] = a;
     }
     if (lane == 0) {
       m_s[r * NW + warp] = m_run[r];
       l_s[r * NW + warp] = l_run[r];
     }
   }
+  __shared__ float s_M[REP], s_l[REP];
+  __shared__ __align__(16) float s_w[REP][NW];
+  __syncthreads();
+  if (warp < REP) {
+    const float mw = lane < NW ? m_s[warp * NW + lane] : -INFINITY;
+    float M = mw;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+    const float f = mw == -INFINITY ? 0.f : __expf(mw - M);  // 0 for a warp without keys
+    const float l = warp_sum_xor(lane < NW ? f * l_s[warp * NW + lane] : 0.f);
+    if (lane < NW) s_w[warp][lane] = f;
+    if (lane == 0) {
+      s_M[warp] = M;
+      s_l[warp] = l;
+    }
+  }
   __syncthreads();
   int* counter = reinterpret_cast<int*>(workspace) + blockIdx.x;
   float* part = reinterpret_cast<float*>(workspace + ATT_COUNTER_BYTES);
   auto part_of = [&](int split, int r) { return part + (static_cast<size_t>(h0 + r) * ATT_MAX_SPLITS + split) * att_part_floats(HD); };
+  auto element = [&](int slot) {  // element of the head that stands in this slot
+    const int k = slot / LPK;
+    return (slot % LPK + LPK * (k / V)) * V + k % V;
+  };
   for (int i = tid; i < REP * HD; i += ATT_THREADS) {
-    const int r = i / HD, d = i - r * HD;
-    float M = -INFINITY, s = 0.f, l = 0.f;
+    const int r = i / HD, slot = i - r * HD;
+    float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) M = fmaxf(M, m_s[r * NW + w]);
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      const float mw = m_s[r * NW + w], f = mw == -INFINITY ? 0.f : __expf(mw - M);  // 0 for a warp without keys
-      s = fmaf(f, red[w * REP * HD + i], s);
-      l = fmaf(f, l_s[r * NW + w], l);
+    for (int w = 0; w < NW; w += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(&s_w[r][w]);
+      s = fmaf(f.x, red[w * REP * HD + i], s);
+      s = fmaf(f.y, red[(w + 1) * REP * HD + i], s);
+      s = fmaf(f.z, red[(w + 2) * REP * HD + i], s);
+      s = fmaf(f.w, red[(w + 3) * REP * HD + i], s);
     }
     if (NSP == 1) {
-      out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(s / l);
+      out[static_cast<size_t>(h0 + r) * HD + element(slot)] = DT<T>::from_f(s / s_l[r]);
     } else {
       float* mine = part_of(sp, r);
-      __stcg(mine + d, s);
-      if (d == 0) {
-        __stcg(mine + HD, M);
-        __stcg(mine + HD + 1, l);
+      __stcg(mine + slot, s);
+      if (slot == 0) {
+        __stcg(mine + HD, s_M[r]);
+        __stcg(mine + HD + 1, s_l[r]);
       }
     }
   }
   if (NSP == 1) return;
   // ---- the split that arrives last merges: out = sum_s e^(m_s - M) acc_s / sum_s e^(m_s - M) l_s
   __shared__ int s_last;
-  __threadfence();
-  __syncthreads();
+  __syncthreads();  // the block's partial results precede thread 0's release
   if (tid == 0) {
-    const int t = atomicAdd(counter, 1);
+    int t;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(t) : "l"(counter) : "memory");
     s_last = t == NSP - 1;
     if (s_last) *counter = 0;  // every other split has arrived: ready for the next launch
   }
   __syncthreads();
   if (!s_last) return;
-  __threadfence();
+  float v[ATT_MAX_SPLITS];  // all loads in flight together, next to those of the weights
+  auto load_parts = [&](int i) {
+    const int r = i / HD;
+    const float* pk = part_of(0, r) + (i - r * HD);
+#pragma unroll
+    for (int k = 0; k < ATT_MAX_SPLITS; ++k) v[k] = k < NSP ? __ldcg(pk + static_cast<size_t>(k) * att_part_floats(HD)) : 0.f;
+  };
+  if (tid < REP * HD) load_parts(tid);
   float* wgt = red;  // [REP][ATT_MAX_SPLITS] weights; behind them the sums of exponentials
   float* den_s = red + REP * ATT_MAX_SPLITS;
   if (warp < REP) {
@@ -307,14 +343,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) k_attn_decode(const T* __restr
   }
   __syncthreads();
   for (int i = tid; i < REP * HD; i += ATT_THREADS) {
-    const int r = i / HD, d = i - r * HD;
-    const float* pk = part_of(0, r) + d;
-    float v[ATT_MAX_SPLITS], num = 0.f;  // all loads in flight together
-#pragma unroll
-    for (int k = 0; k < ATT_MAX_SPLITS; ++k) v[k] = k < NSP ? __ldcg(pk + static_cast<size_t>(k) * att_part_floats(HD)) : 0.f;
+    const int r = i / HD;
+    if (i != tid) load_parts(i);
+    float num = 0.f;
 #pragma unroll
     for (int k = 0; k < ATT_MAX_SPLITS; ++k) num = fmaf(wgt[r * ATT_MAX_SPLITS + k], v[k], num);  // weight 0 beyond NSP
-    out[static_cast<size_t>(h0) * HD + i] = DT<T>::from_f(num / den_s[r]);
+    out[static_cast<size_t>(h0 + r) * HD + element(i - r * HD)] = DT<T>::from_f(num / den_s[r]);
   }
 }
 

@@ -20,7 +20,7 @@ def test_attention_splits(dtype, hd, heads, kv):
     cos, sin = rope_tables(LlamaSkipConfig(head_dim=hd, max_len=max_len), DEV)
     kc, vc, ws = rn(kv, max_len, hd), rn(kv, max_len, hd), attn_workspace(heads, hd, DEV)
     eps = torch.finfo(dtype).eps
-    for pos in (0, 1, 47, 48, 97, 300, 1023, 4097, 8191):
+    for pos in (0, 1, 47, 48, 97, 128, 129, 256, 257, 300, 512, 513, 1023, 1024, 1025, 4097, 8191):  # one block up to two tiles
         qkv = rn((heads + 2 * kv) * hd)
         k0, v0 = kc.clone(), vc.clone()
         out = attn_decode(qkv, cos, sin, torch.tensor([pos], device=DEV), kc, vc, torch.zeros(1, heads * hd, dtype=dtype, device=DEV),
