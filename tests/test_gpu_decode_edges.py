@@ -10,7 +10,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("hd,heads,kv", [(64, 8, 2), (128, 6, 2), (256, 4, 4), (64, 12, 6), (128, 7, 1), (256, 4, 1)])
+@pytest.mark.parametrize("hd,heads,kv", [(64, 8, 2), (128, 6, 2), (256, 4, 4), (64, 12, 6), (128, 7, 1), (256, 4, 1), (64, 32, 8), (128, 32, 4), (256, 32, 8)])
 def test_attention_splits(dtype, hd, heads, kv):
     from sparse_transformers_b200.llama_skip import LlamaSkipConfig, apply_rope, attn_decode, attn_workspace, rope_tables
 
